@@ -85,23 +85,23 @@ void launch_cond_est(const cd* Q, int nang, int n, int ld, int force, int* flag,
 // complex values plus 12 KB in shared memory (227 KB per block).
 constexpr int kMaxBeams = 832;
 
-// K8: Q^{-1} P by blocked Gauss-Jordan with partial pivoting, per flagged angle.
-// scratch: gj_scratch_bytes(nang, n) bytes.  arith: the rounding of the complex
-// multiply-adds:
-//   kGjProductFirst  products formed first, then added (the reference's rounding),
-//                    shared-memory panel and one thread per trailing column (the
-//                    boundary transforms and the bulk solve),
-//   kGjFused         four fused multiply-adds per complex product in the
-//                    row-per-thread panel, the trailing update on the FP64 tensor
-//                    path (the split forms' renormalisations),
-//   kGjFp64Mma       the row-per-thread panel with products formed first, the
-//                    trailing update on the FP64 tensor path (the FP64 form's
-//                    renormalisations).
-// Beyond 640 beams every form takes the shared-memory kernels.
-enum GjArith { kGjProductFirst = 0, kGjFused = 1, kGjFp64Mma = 2 };
+// K8: [Q | P] -> [I | Q^{-1} P] by Gauss-Jordan with partial pivoting, per flagged
+// angle.  scratch: gj_scratch_bytes(nang, n) bytes.  Returns the launches.
+//   kGjProductFirst  shared-memory panels, products formed first, then added (the
+//                    bulk solve, whose ill-conditioned cells follow the reference's
+//                    rounding); Q is left as the elimination leaves it,
+//   kGjFp64, kGjFused  the surface solve: clusters and the FP64 tensor path
+//                    (renorm.cu) up to kGjClusterMaxRows beams; beyond, the
+//                    shared-memory panels with products first (the FP64 form) or
+//                    four fused multiply-adds per complex product (the split forms).
+enum GjArith { kGjProductFirst = 0, kGjFused = 1, kGjFp64 = 2 };
+constexpr int kGjClusterMaxRows = 640;
 size_t gj_scratch_bytes(int nang, int n);
-void launch_gauss_jordan(cd* Q, cd* P, const int* flag, int nang, int n, int ld, void* scratch,
-                         unsigned* status, cudaStream_t st, int arith = kGjProductFirst);
+int launch_gauss_jordan(cd* Q, cd* P, const int* flag, int nang, int n, int ld, void* scratch,
+                        unsigned* status, cudaStream_t st, int arith = kGjProductFirst);
+size_t gj_cluster_scratch_bytes(int nang, int n);
+int launch_gj_cluster(cd* Q, cd* P, const int* flag, int nang, int n, int ld, void* scratch,
+                      unsigned* status, cudaStream_t st);
 
 // RK4 stage combination (rk4_int, surf_rk.f90:27-91); see kernels_f64.cu.
 void launch_rk4_combine(cd* Q, cd* P, cd* Qt, cd* Pt, cd* KP, cd* SQ, cd* SP, int j, double w,

@@ -219,7 +219,6 @@ struct RunState {
   SplitWorkspace sw{};
   int interval = 1;          // renormalisation interval of the growth-bound policy
   long renorms = 0, products = 0, launches = 0, gj_launches = 0;
-  int gj_per = 0;
   bool capturing = false;    // launches go into a CUDA graph: no events on the stream
   long prof_entries = 0;     // event quadruples recorded in profile mode
   long renorm_entries = 0;   // event pairs around renormalisations (profile mode)
@@ -456,7 +455,6 @@ void begin_run(trhepd_context* C, trhepd_problem& Pb, int precision, int nprod_m
         W.split->ensure(split_workspace_bytes(nang, n, C->split_slices, R.nprob)), nang, n,
         C->split_slices, R.status, st, R.nprob);
   R.sw.max_ctas = C->max_ctas;
-  R.gj_per = 2 * ceil_div(n, 16);
   if (C->profile && (int)C->evpool.size() < 4 * nprod_max) {
     while ((int)C->evpool.size() < 4 * nprod_max) {
       cudaEvent_t e;
@@ -488,10 +486,10 @@ void begin_run(trhepd_context* C, trhepd_problem& Pb, int precision, int nprod_m
   }
   // invstransh: Q = I + F^H, P = I - F^H; P <- Q^{-1} P; P <- i P conj(G); Q = I
   launch_invstransh_build(Pb.F.as<cd>(), R.Q, R.P, nang, n, ld, st);
-  launch_gauss_jordan(R.Q, R.P, nullptr, nang, n, ld, R.gjs, R.status, st);
+  R.launches += launch_gauss_jordan(R.Q, R.P, nullptr, nang, n, ld, R.gjs, R.status, st,
+                                    R.split ? kGjFused : kGjFp64);
   launch_invstransh_finish(R.P, R.gam, nang, n, ld, st);
-  launch_set_identity(R.Q, nullptr, nang, n, ld, st);
-  R.launches += 4 + R.gj_per;
+  R.launches += 2;
   if (C->renorm_policy == 1) {
     double kap = Pb.kappa_max + 1.0;
     R.interval = std::max(1, (int)std::floor(C->renorm_tau / (kap * Pb.dz)));
@@ -567,18 +565,16 @@ void renormalise(trhepd_context* C, RunState& R, int l, bool every_slice) {
 void renormalise_launch(trhepd_context* C, RunState& R, bool last, int l, bool every_slice) {
   if (C->renorm_policy == 0 && !every_slice) {
     launch_cond_est(R.Q, R.nang, R.n, R.ld, last ? 1 : 0, R.flags, R.dval, R.st);
-    launch_gauss_jordan(R.Q, R.P, R.flags, R.nang, R.n, R.ld, R.gjs, R.status, R.st,
-                        R.split ? kGjFused : kGjFp64Mma);
-    launch_set_identity(R.Q, R.flags, R.nang, R.n, R.ld, R.st);
-    R.launches += 2 + R.gj_per;
-    R.gj_launches += R.gj_per;
+    const int k = launch_gauss_jordan(R.Q, R.P, R.flags, R.nang, R.n, R.ld, R.gjs, R.status,
+                                      R.st, R.split ? kGjFused : kGjFp64);
+    R.launches += 1 + k;
+    R.gj_launches += k;
     if (!last) ++R.renorms;  // upper bound; per-angle decisions stay on the device
   } else if (last || every_slice || (l % R.interval) == 0) {
-    launch_gauss_jordan(R.Q, R.P, nullptr, R.nang, R.n, R.ld, R.gjs, R.status, R.st,
-                        R.split ? kGjFused : kGjFp64Mma);
-    launch_set_identity(R.Q, nullptr, R.nang, R.n, R.ld, R.st);
-    R.launches += 1 + R.gj_per;
-    R.gj_launches += R.gj_per;
+    const int k = launch_gauss_jordan(R.Q, R.P, nullptr, R.nang, R.n, R.ld, R.gjs, R.status,
+                                      R.st, R.split ? kGjFused : kGjFp64);
+    R.launches += k;
+    R.gj_launches += k;
     if (!last) ++R.renorms;
   }
 }
@@ -591,11 +587,12 @@ void finish_device(trhepd_context* C, trhepd_problem& Pb, RunState& R) {
     launch_strans_build(R.Q, R.P, R.gam, nang, n, ld, st);  // strans + matAdivB2
   else
     launch_stransh_build(R.Q, R.P, R.gam, nang, n, ld, st);
-  launch_gauss_jordan(R.Q, R.P, nullptr, nang, n, ld, R.gjs, R.status, st);
+  R.launches += launch_gauss_jordan(R.Q, R.P, nullptr, nang, n, ld, R.gjs, R.status, st,
+                                    R.split ? kGjFused : kGjFp64);
   launch_check_finite(R.P, (size_t)nang * n * ld, R.status, st);
   launch_intensities(R.P, R.gam, Pb.wnsga2.as<double>(), nang, n, ld, Pb.nb0,
                      Pb.f2.as<double>(), st);
-  R.launches += 3 + R.gj_per;
+  R.launches += 3;
   if (!R.capturing) CK(cudaEventRecord(C->ev1, st));
   CK(cudaGetLastError());
 }
