@@ -13,7 +13,7 @@ from pathlib import Path
 HERE = Path(__file__).resolve().parent
 CSRC = HERE / "csrc"
 OUT = HERE / "_lib" / "libtrhepd_b200.so"
-SOURCES = ["kernels_f64.cu", "renorm.cu", "split_gemm.cu", "bulk.cu", "magnus.cu", "small.cu", "solver.cu",
+SOURCES = ["kernels_f64.cu", "renorm.cu", "convolve.cu", "split_gemm.cu", "bulk.cu", "magnus.cu", "small.cu", "solver.cu",
            "curves.cu", "noalloc.cu", "cholqr.cu",
            "host_model.cpp", "bulk_model.cpp"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]

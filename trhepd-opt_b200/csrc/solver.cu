@@ -20,6 +20,7 @@
 #include "bulk.h"
 #include "magnus.h"
 #include "bulk_model.h"
+#include "convolve.h"
 #include "curves.h"
 #include "host_model.h"
 #include "integrators.h"
@@ -106,7 +107,7 @@ struct trhepd_context {
   std::vector<cudaEvent_t> rnpool;  // profile mode: pairs around renormalisations
   // device buffers (grown on demand, reused across calls)
   DevBuf asf, b, dchg, ghk, z[3], ocr[3], ielm[3], st[3], depth, table, pair;
-  DevBuf Q0, Q1, P, V, D, gam, F, flags, dval, gj, f2, wnsga2, status, split;
+  DevBuf Q0, Q1, P, V, D, gam, F, flags, dval, gj, f2, wnsga2, status, split, spec;
   DevBuf sgh, sgk, simg, snimg, sst;
   DevBuf cva, cvf, cvo;  // rocking-curve convolution of host curves
   DevBuf cerr, cref;     // per-curve errors / distances, reference curves of a comparison
@@ -202,7 +203,7 @@ namespace {
 
 // Device buffers and counters of one integration of a resident problem.
 struct RunState {
-  int n = 0, ns = 0, nv = 0, nang = 0, ld = 0, kpad = 0;
+  int n = 0, ns = 0, nv = 0, nang = 0, ld = 0, kpad = 0, ncol = 0;
   bool split = false;
   int split_variant = kSplitPersistent;
   cudaStream_t st = nullptr;
@@ -227,18 +228,23 @@ struct RunState {
   int nprob = 1;             // stacked problems (see trhepd_problem::nprob)
   const TableEntry* const* tables = nullptr;
   StackedRows sr{};          // rows and stage-matrix stride per stacked problem
+  bool conv = false;         // stage products as convolutions (convolve.h)
+  ConvStages cs{};           // their constant arguments
+  const int* centry = nullptr;
+  cd* spec = nullptr;        // spectra of columns spec_col .. spec_col + spec_n - 1
+  int spec_col = 0, spec_n = 0, spec_cap = 0;
 };
 
 // The device buffers one integration works in: the context's (one solve at a
 // time) or a problem's own (problems solved together in a batch).
 struct Workspace {
-  DevBuf *Q0, *Q1, *P, *V, *flags, *dval, *gj, *status, *split;
+  DevBuf *Q0, *Q1, *P, *V, *flags, *dval, *gj, *status, *split, *spec;
 };
 struct OwnWorkspace {
-  DevBuf Q0, Q1, P, V, flags, dval, gj, status, split;
-  Workspace view() { return {&Q0, &Q1, &P, &V, &flags, &dval, &gj, &status, &split}; }
+  DevBuf Q0, Q1, P, V, flags, dval, gj, status, split, spec;
+  Workspace view() { return {&Q0, &Q1, &P, &V, &flags, &dval, &gj, &status, &split, &spec}; }
   void release() {
-    for (DevBuf* b : {&Q0, &Q1, &P, &V, &flags, &dval, &gj, &status, &split}) b->release();
+    for (DevBuf* b : {&Q0, &Q1, &P, &V, &flags, &dval, &gj, &status, &split, &spec}) b->release();
   }
 };
 
@@ -255,6 +261,8 @@ struct trhepd_problem {
   int nprob = 1;
   const TableEntry* const* tables = nullptr;
   std::vector<int> pair_host;  // the beam-pair map, to recognise problems that stack
+  ConvGrid grid;               // m = 0: stage products as dense products only
+  DevBuf ccell, cmask, centry, cD;
   Integrator I{};
   double dz = 0, kappa_max = 0;
   int ncol = 0;
@@ -296,12 +304,13 @@ struct trhepd_problem {
     return graphs.back();
   }
   size_t bytes() const {
-    return table.n + pair.n + gam.n + D.n + F.n + wnsga2.n + f2.n + f2ref.n;
+    return table.n + pair.n + gam.n + D.n + F.n + wnsga2.n + f2.n + f2ref.n + cD.n;
   }
   void release() {
     drop_graph();
     own.release();
-    for (DevBuf* b : {&table, &pair, &gam, &D, &F, &wnsga2, &f2, &dang, &conv, &f2ref})
+    for (DevBuf* b : {&table, &pair, &gam, &D, &F, &wnsga2, &f2, &dang, &conv, &f2ref, &ccell,
+                      &cmask, &centry, &cD})
       b->release();
   }
 };
@@ -338,6 +347,20 @@ void prepare(trhepd_context* C, const SolveArgs& A, trhepd_problem& Pb) {
     }
   upload(Pb.pair, pair, st);
   Pb.pair_host = pair;
+  // the beams' index grid, if the pair map is a function of the beam difference; that the
+  // table agrees for differences met in both beam orders is checked on the device
+  Pb.grid = conv_grid(n, A.ih, A.ik, pair.data());
+  int* d_bad = nullptr;
+  int bad = 0;
+  if (Pb.grid.m) {
+    upload(Pb.ccell, Pb.grid.cell, st);
+    upload(Pb.cmask, Pb.grid.mask, st);
+    upload(Pb.centry, Pb.grid.entry, st);
+    d_bad = (int*)C->sgk.ensure(16);
+    CK(cudaMemsetAsync(d_bad, 0, sizeof(int), st));
+    const int* tw = upload(C->sgh, Pb.grid.twins, st);
+    launch_conv_check(table, Pb.ncol, nv, tw, (int)Pb.grid.twins.size() / 2, d_bad, st);
+  }
 
   // angle schedule (surflf.f90:43-92)
   const bool ng_outer = A.ng > A.naz;
@@ -410,13 +433,38 @@ void prepare(trhepd_context* C, const SolveArgs& A, trhepd_problem& Pb) {
   upload(Pb.F, F, st);
   upload(Pb.wnsga2, wnsga2, st);
   Pb.f2.ensure((size_t)nang * n * sizeof(double));
+  if (Pb.grid.m) {
+    const int m = Pb.grid.m;
+    std::vector<double> Dg((size_t)nang * Pb.grid.sy * m, 0.0);
+    for (int t = 0; t < nang; ++t)
+      for (int i = 0; i < n; ++i) {
+        const int c = Pb.grid.cell[i];
+        Dg[((size_t)t * Pb.grid.sy + (c >> 8)) * m + (c & 255)] = Dm[(size_t)t * ld + i].x;
+      }
+    upload(Pb.cD, Dg, st);
+    CK(cudaMemcpyAsync(&bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    if (bad) Pb.grid.m = 0;
+  }
 }
 
 
 // Buffers, the boundary transform invstransh (matcomp.f90:140-172) and the
 // renormalisation schedule; Q = I and P = P0 afterwards.
 Workspace context_workspace(trhepd_context* C) {
-  return {&C->Q0, &C->Q1, &C->P, &C->V, &C->flags, &C->dval, &C->gj, &C->status, &C->split};
+  return {&C->Q0, &C->Q1, &C->P, &C->V, &C->flags, &C->dval, &C->gj, &C->status, &C->split,
+          &C->spec};
+}
+
+// Whether the stage products of a solve are convolutions over the beam grid.  Against the
+// dense FP64 products they always pay where conv_grid returns a grid (n = 521, 16 angles:
+// 0.68 -> 0.17 ms per stage; n = 95, 61 angles: 56 -> 14.5 us).  Against the digit products
+// with 5 slices too (n = 521, 31 angles: 0.37 -> 0.31 ms; n = 191, 61 angles: 103 -> 54
+// us); 3 and 4 slices have 6 and 10 slice pairs instead of 15 and stay ahead on the
+// largest grids.
+bool use_convolution(const trhepd_context* C, const trhepd_problem& Pb, bool split) {
+  if (!Pb.grid.m || Pb.I.family > kRk4) return false;
+  return !split || C->split_slices >= 5 || Pb.grid.m <= 20;
 }
 
 void begin_run(trhepd_context* C, trhepd_problem& Pb, int precision, int nprod_max, RunState& R,
@@ -424,6 +472,7 @@ void begin_run(trhepd_context* C, trhepd_problem& Pb, int precision, int nprod_m
   R.n = Pb.n;
   R.ns = Pb.ns;
   R.nv = Pb.nv;
+  R.ncol = Pb.ncol;
   R.nang = Pb.nang;
   R.ld = Pb.ld;
   R.kpad = Pb.ld;
@@ -435,8 +484,10 @@ void begin_run(trhepd_context* C, trhepd_problem& Pb, int precision, int nprod_m
   const int n = R.n, nang = R.nang, ld = R.ld;
   cudaStream_t st = R.st;
   R.sbytes = (size_t)nang * n * ld * sizeof(cd);
+  R.split = precision == TRHEPD_SPLIT_BF16 || precision == TRHEPD_SPLIT_INT8;
+  R.conv = use_convolution(C, Pb, R.split);
   R.Q = (cd*)W.Q0->ensure(R.sbytes);
-  R.Qn = (cd*)W.Q1->ensure(R.sbytes);
+  if (!R.conv) R.Qn = (cd*)W.Q1->ensure(R.sbytes);  // the dense products' second Q
   R.P = (cd*)W.P->ensure(R.sbytes);
   R.nprob = Pb.nprob;
   R.tables = Pb.tables;
@@ -446,15 +497,34 @@ void begin_run(trhepd_context* C, trhepd_problem& Pb, int precision, int nprod_m
   R.dval = (double*)W.dval->ensure(std::max(nang, 4) * sizeof(double));
   R.gjs = W.gj->ensure(gj_scratch_bytes(nang, n));
   R.status = (unsigned*)W.status->ensure(16);
-  R.split = precision == TRHEPD_SPLIT_BF16 || precision == TRHEPD_SPLIT_INT8;
   R.split_variant = (precision == TRHEPD_SPLIT_INT8) ? kSplitInt8 : C->split_variant;
   if (precision == TRHEPD_SPLIT_BF16 && C->split_slices > 5)
     throw std::invalid_argument("the BF16 split form takes 3 to 5 slices");
-  if (R.split)
+  if (R.split && !R.conv)
     R.sw = split_workspace_carve(
         W.split->ensure(split_workspace_bytes(nang, n, C->split_slices, R.nprob)), nang, n,
         C->split_slices, R.status, st, R.nprob);
   R.sw.max_ctas = C->max_ctas;
+  if (R.conv) {
+    // spectra of a stretch of stage columns at a time (64 MB, at least two slices')
+    const size_t per = (size_t)R.nprob * conv_spectrum_elems(Pb.grid.m) * sizeof(cd);
+    R.spec_cap = (int)std::max<size_t>(2, (size_t(64) << 20) / (per * Pb.I.s)) * Pb.I.s;
+    R.spec_cap = std::min(R.spec_cap, ceil_div(Pb.ncol, Pb.I.s) * Pb.I.s);
+    R.spec = (cd*)W.spec->ensure((size_t)R.spec_cap * per);
+    R.centry = Pb.centry.as<int>();
+    R.cs = ConvStages{};
+    R.cs.spec_stride = (size_t)R.spec_cap * conv_spectrum_elems(Pb.grid.m);
+    R.cs.cell = Pb.ccell.as<int>();
+    R.cs.mask = Pb.cmask.as<unsigned>();
+    R.cs.D = Pb.cD.as<double>();
+    R.cs.n = n;
+    R.cs.ld = ld;
+    R.cs.rows = nang * n;
+    R.cs.rows_b = (nang / R.nprob) * n;
+    R.cs.m = Pb.grid.m;
+    R.cs.sx = Pb.grid.sx;
+    R.cs.sy = Pb.grid.sy;
+  }
   if (C->profile && (int)C->evpool.size() < 4 * nprod_max) {
     while ((int)C->evpool.size() < 4 * nprod_max) {
       cudaEvent_t e;
@@ -472,7 +542,7 @@ void begin_run(trhepd_context* C, trhepd_problem& Pb, int precision, int nprod_m
   if (!R.capturing) CK(cudaEventRecord(C->ev0, st));
   CK(cudaMemsetAsync(R.status, 0, 16, st));
   CK(cudaMemsetAsync(R.Q, 0, R.sbytes, st));
-  CK(cudaMemsetAsync(R.Qn, 0, R.sbytes, st));
+  if (R.Qn) CK(cudaMemsetAsync(R.Qn, 0, R.sbytes, st));
   CK(cudaMemsetAsync(R.P, 0, R.sbytes, st));
   if (Pb.I.gs) {
     // rk4_intgs (surf_rk.f90:106-109): invstrans, CholeskyQR of every angle, the
@@ -509,6 +579,40 @@ void reorthogonalise(trhepd_context* C, RunState& R) {
   if (ev) {
     CK(cudaEventRecord(ev[1], R.st));
     ++R.renorm_entries;
+  }
+}
+
+// `nstage` convolution stages from table column `col` on Q and P in place: stage i has the
+// coefficients of k = i mod s (cb0 in place of the first), P += cb (Q M), Q += ca P.
+void conv_stages(trhepd_context* C, RunState& R, cd* Q, cd* P, int col, int nstage, int s,
+                 double cb0, const double* cb, const double* ca) {
+  R.cs.Q = Q;
+  R.cs.P = P;
+  R.cs.s = s;
+  for (int k = 0; k < s; ++k) {
+    R.cs.cb[k] = cb[k];
+    R.cs.ca[k] = ca[k];
+  }
+  for (int done = 0; done < nstage;) {  // a launch ends with the spectra at hand
+    int at = col + done;
+    if (at < R.spec_col || at >= R.spec_col + R.spec_n) {
+      R.spec_col = at;
+      R.spec_n = std::min(R.spec_cap, R.ncol - at);
+      launch_conv_spectra(R.table, R.tables, R.nprob, at, R.spec_n, R.nv, R.centry, R.cs.m,
+                          R.cs.sx, R.cs.sy, R.spec, R.cs.spec_stride, R.st);
+      R.launches += 1;
+    }
+    R.cs.nstage = std::min(nstage - done, R.spec_col + R.spec_n - at);
+    R.cs.cb0 = done == 0 ? cb0 : cb[0];
+    R.cs.spec = R.spec + (size_t)(at - R.spec_col) * conv_spectrum_elems(R.cs.m);
+    const cudaEvent_t* ev = C->profile ? &C->evpool[4 * R.prof_entries] : nullptr;
+    for (int e = 0; ev && e < 2; ++e) CK(cudaEventRecord(ev[e], R.st));
+    launch_conv_stages(R.cs, C->max_ctas, R.st);
+    for (int e = 2; ev && e < 4; ++e) CK(cudaEventRecord(ev[e], R.st));
+    if (ev) ++R.prof_entries;
+    R.launches += 1;
+    R.products += R.cs.nstage;
+    done += R.cs.nstage;
   }
 }
 
@@ -686,7 +790,22 @@ void run_rkn(trhepd_context* C, trhepd_problem& Pb, int precision, RunState& R) 
     finish_device(C, Pb, R);
     return;
   }
-  for (int l = 1; l <= R.ns; ++l) {
+  if (R.conv) {
+    // all stages up to the next renormalisation in one launch; Q = I enters as data
+    double cb[11], ca[11];
+    for (int k = 0; k < I.s; ++k) {
+      cb[k] = (k == 0 ? 2.0 : 1.0) * I.bab[2 * k] * dz;
+      ca[k] = I.bab[2 * k + 1] * dz;
+    }
+    const int group = (C->renorm_policy == 0 || every_slice) ? 1 : R.interval;
+    for (int l0 = 0; l0 < R.ns; l0 += group) {
+      const int l1 = std::min(l0 + group, R.ns);
+      conv_stages(C, R, R.Q, R.P, I.s * l0, I.s * (l1 - l0), I.s,
+                  l0 == 0 ? I.bab[0] * dz : cb[0], cb, ca);
+      renormalise(C, R, l1, every_slice);
+    }
+  }
+  for (int l = 1; l <= R.ns && !R.conv; ++l) {
     for (int k = 1; k <= I.s; ++k) {
       const int col = I.s * (l - 1) + k - 1;
       const double ca = I.bab[2 * k - 1] * dz;
@@ -725,7 +844,17 @@ void run_lf(trhepd_context* C, trhepd_problem& Pb, int precision, RunState& R) {
   gather(R, 0, false);  // any finite stage matrix: cb = 0 below
   launch_stage_identity(R.Q, R.P, R.V, R.D, R.nang, R.n, R.ld, 0.0, 0.5 * dz, R.st);
   R.launches += 1;
-  for (int l = 1; l <= R.ns; ++l) {
+  if (R.conv) {
+    const int group = C->renorm_policy == 0 ? 1 : R.interval;
+    for (int l0 = 0; l0 < R.ns;) {  // the last slice, with its half step, on its own
+      const int l1 = l0 + 1 == R.ns ? R.ns : std::min({(l0 / group + 1) * group, R.ns - 1});
+      const double dz2 = l1 == R.ns ? dz / 2 : dz;
+      conv_stages(C, R, R.Q, R.P, l0, l1 - l0, 1, dz, &dz, &dz2);
+      renormalise(C, R, l1, false);
+      l0 = l1;
+    }
+  }
+  for (int l = 1; l <= R.ns && !R.conv; ++l) {
     const double dz2 = (l == R.ns) ? dz / 2 : dz;
     gather(R, l - 1, R.split);
     stage_product(C, R, R.Q, R.P, R.Qn, dz, dz2);
@@ -758,8 +887,13 @@ void run_rk4(trhepd_context* C, trhepd_problem& Pb, int precision, RunState& R) 
     const double w[4] = {1.0, 2.0, 2.0, 1.0};
     const double step[4] = {half, half, dz, 0.0};
     for (int j = 0; j < 4; ++j) {
-      gather(R, cols[j], R.split);
-      stage_product(C, R, j == 0 ? R.Q : Qt, KP, R.Qn, 1.0, 0.0);
+      if (R.conv) {
+        const double one = 1.0, zero = 0.0;
+        conv_stages(C, R, j == 0 ? R.Q : Qt, KP, cols[j], 1, 1, one, &one, &zero);
+      } else {
+        gather(R, cols[j], R.split);
+        stage_product(C, R, j == 0 ? R.Q : Qt, KP, R.Qn, 1.0, 0.0);
+      }
       launch_rk4_combine(R.Q, R.P, Qt, Pt, KP, SQ, SP, j, w[j], step[j], dz / 6, R.nang, R.n,
                          R.ld, R.st);
       R.launches += 1;
@@ -892,7 +1026,7 @@ void run_device(trhepd_context* C, trhepd_problem& Pb, int precision, RunState& 
 // The context buffers a solve's launches address; a graph stays valid while they do.
 std::vector<void*> buffer_signature(const trhepd_context* C) {
   std::vector<void*> s = {C->Q0.p, C->Q1.p, C->P.p, C->V.p, C->flags.p, C->dval.p,
-                          C->gj.p, C->status.p, C->split.p};
+                          C->gj.p, C->status.p, C->split.p, C->spec.p};
   for (const DevBuf& b : C->rk) s.push_back(b.p);
   for (const DevBuf& b : C->mg) s.push_back(b.p);
   return s;
@@ -984,7 +1118,7 @@ void run_checked(trhepd_context* C, trhepd_problem& Pb, int precision) {
 bool stackable(const trhepd_problem& a, const trhepd_problem& b) {
   return a.n == b.n && a.ns == b.ns && a.dz == b.dz && a.int_method == b.int_method &&
          a.nang == b.nang && a.nv == b.nv && a.ncol == b.ncol && a.nb0 == b.nb0 &&
-         a.pair_host == b.pair_host;
+         a.grid.m == b.grid.m && a.grid.cell == b.grid.cell && a.pair_host == b.pair_host;
 }
 
 // One integration of a stacked group; the intensities go back to each problem.
@@ -1009,10 +1143,15 @@ void solve_stacked(trhepd_context* C, const std::vector<trhepd_problem*>& g, int
   for (const trhepd_problem* p : g) M.kappa_max = std::max(M.kappa_max, p->kappa_max);
   M.pair.p = p0.pair.p;    // borrowed (shared beam-pair map)
   M.table.p = p0.table.p;  // borrowed (the tables array holds every problem's)
+  M.grid = p0.grid;
+  M.ccell.p = p0.ccell.p;  // borrowed, as the next two (the same beam grid)
+  M.cmask.p = p0.cmask.p;
+  M.centry.p = p0.centry.p;
   DevBuf tabs;
   auto unborrow = [&]() {
     M.pair.p = nullptr;
     M.table.p = nullptr;
+    M.ccell.p = M.cmask.p = M.centry.p = nullptr;
     M.release();
     tabs.release();
   };
@@ -1029,6 +1168,7 @@ void solve_stacked(trhepd_context* C, const std::vector<trhepd_problem*>& g, int
     stack(M.D, &trhepd_problem::D, (size_t)na * ld * sizeof(cd));
     stack(M.F, &trhepd_problem::F, (size_t)na * n * n * sizeof(cd));
     stack(M.wnsga2, &trhepd_problem::wnsga2, (size_t)na * sizeof(double));
+    if (M.grid.m) stack(M.cD, &trhepd_problem::cD, (size_t)na * M.grid.sy * M.grid.m * sizeof(double));
     M.f2.ensure((size_t)M.nang * n * sizeof(double));
     RunState R;
     run_device(C, M, precision, R);
