@@ -1,23 +1,28 @@
 // Fused small-beam RKN integration (hp_int_spa, sim-trhepd-rheed/src/surf_prkn.f90:278-330).
 //
-// For N <= 64 beams a whole angle fits one SM: Q = X^H, P = Y^H and the stage
-// matrix (NP x NP complex each, NP = N rounded up to 16) stay in shared memory
-// for all s*ns stages, so the solve is one launch (one CTA per angle) instead of
-// several launches per stage.  Per stage:
-//   * the next stage column's matrix entries are loaded into registers (one fixed
-//     set of (k, j) positions per thread, beam-pair indices held in registers)
-//     while the current product runs;
-//   * the product Q V runs on the FP64 tensor cores (mma.sync m16n8k4, 4 real
-//     MMAs per complex product), one warp per 16 rows x NP/2 columns;
+// For N <= 64 beams a whole angle fits one SM, so the solve is one launch, one CTA of
+// four warps per angle, through all s*ns stages:
+//   * the stage columns of the potential table (nv entries) are copied into shared memory
+//     three stages ahead; the product reads the matrix entries
+//     straight from it (V(k, j) is an entry of pair(k, j), conjugated or not: the
+//     fragments' entry numbers stay packed in registers), so no stage matrix is formed;
+//   * the product Q V runs on the FP64 tensor cores (mma.sync m16n8k4 on (re, im) column
+//     pairs): a warp owns whole 16-row tiles times every WC-th group of four columns, so
+//     the four schedulers get equal shares, and a lane holds whole complex elements;
 //   * the epilogue is the RKN update of the stacked path: P += cb (Q V + Q o D_a),
-//     Q <- Q + ca P (the identity stages Q = I are elementwise);
+//     Q <- Q + ca P; P stays in registers (shared memory beyond 48 beams); Q = I enters
+//     as data;
 //   * at the end of a slice the renormalisation (policy 0: Gershgorin estimate
 //     cond_est, matcomp.f90:498-528, > 1e3; policy 1: every `interval` slices;
-//     always on the last) is an in-place Gauss-Jordan of [Q | P] with partial
-//     pivoting on max |re| + |im| (matAbdivB, matcomp.f90:53-69), then Q = I.
-// The stage order, merged half kicks and coefficients are those of run_rkn.
+//     always on the last) is a Gauss-Jordan elimination of [Q | P] (matAbdivB,
+//     matcomp.f90:53-69) with implicit pivoting in 16-column sub-panels, as renorm.cu:
+//     the panel's rows in registers, its E in the panel's own columns of Q, the other
+//     columns updated by MMAs.
+// The stage order, merged half kicks and coefficients are those of run_rkn.  What bounds
+// it: at N = 47 the FP64 pipe (6.9 K clocks a product), at N = 23 the chain of barriers,
+// shared-memory latency and 1.2 K clocks of MMAs.
 // One launch can carry several problems (their own tables, beam counts up to
-// the launch's NP, slice counts and renormalisation intervals): each CTA finds
+// the launch's limit, slice counts and renormalisation intervals): each CTA finds
 // its problem in the launch parameters.
 #include <cuda_runtime.h>
 
@@ -30,184 +35,276 @@
 namespace trhepd {
 namespace fused {
 
-template <int NP>
+constexpr int kThreads = 128;
+constexpr int kTabBufs = 4;  // table columns in flight where shared memory allows
+
+// RT row tiles; GW column groups per warp.
+template <int RT, int GW>
 struct Cfg {
-  static constexpr int WARPS = NP / 8;              // NP/16 row tiles x 2 column halves
-  static constexpr int THREADS = 32 * WARPS;
-  static constexpr int QSTR = NP + 4;               // 4 mod 8 complex: conflict-free A reads
-  static constexpr int PSTR = NP + 4;
-  static constexpr int VSTR = NP + 2;               // 2 mod 8 complex: conflict-free B reads
-  static constexpr int NT8 = NP / 16;               // 8-wide column tiles per warp
-  static constexpr int GATHER = NP * NP / THREADS;  // stage-matrix entries per thread
-  static constexpr size_t SMEM = (size_t)(NP * QSTR + NP * PSTR + NP * VSTR) * sizeof(cd);
+  static constexpr int NP = 16 * RT;
+  static constexpr int WC = RT == 2 ? 2 : 4;        // warps along the columns
+  static constexpr int WR = 4 / WC;                 // and along the row tiles
+  static constexpr int TW = RT / WR;                // row tiles per warp
+  static constexpr int KS = 4 * RT;                 // k steps of a product
+  static constexpr bool PREG = RT <= 3;             // P in registers
+  static constexpr int QB = RT <= 2 ? 2 : 1;        // Q buffers (one barrier per stage less)
+  static constexpr int STR = NP + 4;                // 4 mod 8 complex: conflict-free fragments
+  static constexpr int MINB = RT <= 2 ? 3 : RT == 3 ? 2 : 1;
+  // complex values of Q, P and the pivot rows, and the fragment codes (8 bytes per lane
+  // and k step)
+  static constexpr size_t elems =
+      (size_t)(QB + (PREG ? 0 : 1)) * NP * STR + 16 * STR + KS * kThreads / 2;
 };
 
-__device__ __forceinline__ void fdmma(double& c0, double& c1, double& c2, double& c3, double a0,
-                                      double a1, double b0) {
+__device__ __forceinline__ unsigned smem_addr(const void* p) {
+  return (unsigned)__cvta_generic_to_shared(p);
+}
+// Waits for a phase of a barrier, two seconds at most.
+__device__ __forceinline__ bool wait_parity(const unsigned long long* bar, int parity) {
+  unsigned long long t0 = 0;
+  for (unsigned it = 0;; ++it) {
+    unsigned ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_addr(bar)), "r"(parity)
+        : "memory");
+    if (ok) return true;
+    if ((it & 255) == 255) {
+      unsigned long long t;
+      asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+      if (t0 == 0) t0 = t;
+      else if (t - t0 > 2000000000ull) return false;
+    }
+  }
+}
+
+__device__ __forceinline__ void fmma(cd& c0, cd& c1, double a0, double a1, double b0) {
   asm volatile(
       "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, "
       "{%0,%1,%2,%3};\n"
-      : "+d"(c0), "+d"(c1), "+d"(c2), "+d"(c3)
+      : "+d"(c0.x), "+d"(c0.y), "+d"(c1.x), "+d"(c1.y)
       : "d"(a0), "d"(a1), "d"(b0));
 }
 
-template <int NP>
-__global__ void __launch_bounds__(Cfg<NP>::THREADS)
-    k_fused_rkn(const __grid_constant__ FusedLaunch L) {
-  using C = Cfg<NP>;
+template <int RT, int GW>
+__global__ void __launch_bounds__(kThreads, Cfg<RT, GW>::MINB)
+    k_fused_rkn(const __grid_constant__ FusedLaunch L, int nbuf, int tab_stride) {
+  using C = Cfg<RT, GW>;
+  constexpr int NP = C::NP, STR = C::STR, TW = C::TW;
   // this CTA's problem: the last whose first CTA is <= blockIdx.x
   int pi = 0;
   for (int q = 1; q < L.nprob; ++q)
     if (L.p[q].first_cta <= (int)blockIdx.x) pi = q;
   const FusedProblem& a = L.p[pi];
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  cd* Qs = reinterpret_cast<cd*>(smem_raw);
-  cd* Ps = Qs + NP * C::QSTR;
-  cd* Vs = Ps + NP * C::PSTR;
-  __shared__ double red_d[2][C::WARPS];
-  __shared__ int piv_sh, renorm_sh;
+  cd* Qs = reinterpret_cast<cd*>(smem_raw);             // the current Q
+  cd* Qo = Qs + (C::QB - 1) * NP * STR;                 // the other (the same for QB = 1)
+  cd* const Ps = Qs + C::QB * NP * STR;                 // PREG = false only
+  cd* const c1s = Ps + (C::PREG ? 0 : NP * STR);        // 16 pivot rows
+  uint2* const codes = reinterpret_cast<uint2*>(c1s + 16 * STR);  // [KS][kThreads]
+  cd* const tab = c1s + 16 * STR + C::KS * kThreads / 2;          // [nbuf][tab_stride]
+  __shared__ double csum[kThreads];
+  __shared__ double red_d[2][4];
+  __shared__ unsigned keys[2][32];
+  __shared__ cd urow[2][16];
+  __shared__ int order[NP], piv[NP], renorm_sh;
+  __shared__ signed char slot[NP];
+  __shared__ __align__(8) unsigned long long bars[kTabBufs];
+  const unsigned full = 0xffffffffu;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int g = lane >> 2, t = lane & 3;
-  const int n = a.n, ld = a.ld, ang = blockIdx.x - a.first_cta;
-  cd* Qg = a.Q + (size_t)ang * n * ld;
-  cd* Pg = a.P + (size_t)ang * n * ld;
-  const cd* Dg = a.D + (size_t)ang * ld;
+  const int gq = lane >> 2, t4 = lane & 3;
+  const int wr = warp / C::WC, wc = warp % C::WC;
+  const int n = a.n, ld = a.ld, nv = a.nv, ang = blockIdx.x - a.first_cta;
+  const int row0 = wr * TW * 16 + gq;                   // rows row0 + 16 i + 8 h
+  auto col = [&](int j) { return 4 * (j * C::WC + wc) + t4; };
+  cd* const Qg = a.Q + (size_t)ang * n * ld;
+  cd* const Pg = a.P + (size_t)ang * n * ld;
 
-  for (int e = tid; e < NP * NP; e += C::THREADS) {
-    const int i = e / NP, j = e % NP;
-    cd q = cd{0.0, 0.0}, p = cd{0.0, 0.0};
-    if (i < n && j < n) {
-      q = Qg[(size_t)i * ld + j];
-      p = Pg[(size_t)i * ld + j];
-    }
-    Qs[i * C::QSTR + j] = q;
-    Ps[i * C::PSTR + j] = p;
+  cd preg[C::PREG ? TW * 2 * GW : 1];
+  auto P = [&](int i, int h, int j) -> cd& {
+    if constexpr (C::PREG) return preg[(i * 2 + h) * GW + j];
+    else return Ps[(row0 + 16 * i + 8 * h) * STR + col(j)];
+  };
+  for (int e = tid; e < NP * STR; e += kThreads) {
+    const int i = e / STR, j = e % STR;
+    const bool ok = i < n && j < n;
+    Qs[e] = ok ? Qg[(size_t)i * ld + j] : cd{0.0, 0.0};
+    if (C::QB == 2) Qo[e] = cd{0.0, 0.0};
   }
-  // this thread's stage-matrix positions: table index (>= 0), -2 diagonal, -1 zero
-  int pidx[C::GATHER];
-  unsigned upper = 0;
+  double dreg[GW];
 #pragma unroll
-  for (int m = 0; m < C::GATHER; ++m) {
-    const int e = tid + m * C::THREADS, k = e / NP, j = e % NP;
-    pidx[m] = -1;
-    if (k < n && j < n) {
-      if (k == j) {
-        pidx[m] = -2;
-      } else {
-        pidx[m] = a.pair[k * n + j];
-        if (k < j) upper |= 1u << m;
+  for (int j = 0; j < GW; ++j) {
+    dreg[j] = col(j) < n ? a.D[(size_t)ang * ld + col(j)].x : 0.0;  // D = -gamma^2 is real
+#pragma unroll
+    for (int i = 0; i < TW; ++i)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int r = row0 + 16 * i + 8 * h;
+        P(i, h, j) = (r < n && col(j) < n) ? Pg[(size_t)r * ld + col(j)] : cd{0.0, 0.0};
       }
-    }
   }
-  // row tile and column half of this warp; D of its epilogue columns
-  const int m0 = (warp >> 1) * 16, c0 = (warp & 1) * (NP / 2);
-  const bool active = m0 < n && c0 < n;
-  const int kmax = ((n + 3) / 4) * 4;
-  cd dreg[C::NT8][2];
+  // The B fragments' matrix entries: lane (g, t) of k step ks and group j takes V(4 ks + t,
+  // 4 cg + g / 2), as -V: an upper entry (k < j, and the diagonal's entry 0) is conj(u), a
+  // lower one w, so only the imaginary part can change sign.  Even lanes use (re, -im) as
+  // the two k rows, odd ones (im, re): 15 bits of position (16-byte words of the table
+  // column; the zero entry is nv) and the sign.
+  for (int ks = 0; ks < C::KS; ++ks) {
+    unsigned code[4];
 #pragma unroll
-  for (int nt = 0; nt < C::NT8; ++nt)
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int j = c0 + nt * 8 + 2 * t + h;
-      dreg[nt][h] = (j < n) ? Dg[j] : cd{0.0, 0.0};
-    }
-
-  cd vbuf[C::GATHER];
-  auto load_col = [&](int col) {
-    const TableEntry* tc = a.table + (size_t)col * a.nv;
-#pragma unroll
-    for (int m = 0; m < C::GATHER; ++m) {
-      const int p = pidx[m];
-      cd v = cd{0.0, 0.0};
-      if (p >= 0) {
-        v = ((upper >> m) & 1u) ? -conj(tc[p].u) : -tc[p].w;
-      } else if (p == -2) {
-        v = -conj(tc[0].u);
+    for (int j = 0; j < 4; ++j) {
+      const int k = 4 * ks + t4, c = 4 * (j * C::WC + wc) + (gq >> 1);
+      unsigned pos = 2 * nv, lower = 0;
+      if (j < GW && k < n && c < n) {
+        lower = k > c;
+        pos = 2 * (k == c ? 0 : a.pair[k * n + c]) + lower;
       }
-      vbuf[m] = v;
+      code[j] = pos | ((gq & 1) ? 1u - lower : lower) << 15;
+    }
+    codes[ks * kThreads + tid] = make_uint2(code[0] | code[1] << 16, code[2] | code[3] << 16);
+  }
+  const int ng = (n + 3) / 4;  // column groups (and k steps) that hold beams
+  for (int b = 0; b < nbuf; ++b)
+    if (tid < 2) tab[b * tab_stride + 2 * nv + tid] = cd{0.0, 0.0};
+  const int s = L.s, ns = a.ns;
+  const double dz = a.dz;
+  // The next column of the table into the next buffer: one bulk copy by thread 0 (16-byte
+  // copies by every thread took 500 clocks of a stage).  Every issued column is consumed.
+  const int ncol = s * ns + 1;
+  if (tid == 0) {
+    for (int b = 0; b < nbuf; ++b)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&bars[b])) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  int issued = 0, in = 0;           // columns on their way or consumed (thread 0)
+  int consumed = 0, out = 0, parity = 0;
+  bool dead = false;                // a copy that never came: reported, not waited for again
+  auto fetch = [&]() {
+    if (tid == 0 && issued < ncol && !dead) {
+      const unsigned bar = smem_addr(&bars[in]), bytes = 32u * nv;
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
+                   : "memory");
+      asm volatile(
+          "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+          ::"r"(smem_addr(tab + in * tab_stride)), "l"(a.table + (size_t)issued * nv), "r"(bytes),
+          "r"(bar)
+          : "memory");
+      in = in + 1 < nbuf ? in + 1 : 0;
+      ++issued;
     }
   };
-  auto store_col = [&]() {
-#pragma unroll
-    for (int m = 0; m < C::GATHER; ++m) {
-      const int e = tid + m * C::THREADS;
-      Vs[(e / NP) * C::VSTR + (e % NP)] = vbuf[m];
+  auto arrived = [&]() {  // waits for the next column
+    if (!dead && !wait_parity(&bars[out], parity)) {
+      dead = true;
+      atomicOr(a.status, kStatusTimeout);
+    }
+    ++consumed;
+    if (++out == nbuf) {
+      out = 0;
+      parity ^= 1;
     }
   };
-  // P += cb (V + diag(D)), Q = I + ca P  (stage with Q = I)
-  auto identity_stage = [&](double cb, double ca) {
-    for (int e = tid; e < n * n; e += C::THREADS) {
-      const int i = e / n, j = e % n;
-      cd m = Vs[i * C::VSTR + j];
-      if (i == j) m = m + Dg[j];
-      const cd p = Ps[i * C::PSTR + j] + cb * m;
-      Ps[i * C::PSTR + j] = p;
-      cd q = ca * p;
-      if (i == j) q.x += 1.0;
-      Qs[i * C::QSTR + j] = q;
-    }
-  };
-  // P += cb (Q V + Q o D), Q <- Q + ca P; the caller has synchronised; returns
-  // after the product phase's barrier, with the update written (no trailing barrier)
-  auto product_stage = [&](double cb, double ca) {
-    double cr[C::NT8][4], ci[C::NT8][4];
+  for (int c = 0; c < max(nbuf - 1, 1); ++c) fetch();
+  // P += cb (Q V + Q o D), Q <- Q + ca P with the next table column; ends without a barrier
+  auto stage = [&](double cb, double ca) {
+    const cd* tc = tab + out * tab_stride;
+    arrived();
+    __syncthreads();  // Q is there too
+    if (nbuf > 1) fetch();
+    cd acc[TW][2][GW];
 #pragma unroll
-    for (int nt = 0; nt < C::NT8; ++nt)
+    for (int i = 0; i < TW; ++i)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) cr[nt][e] = ci[nt][e] = 0.0;
-    if (active) {
-      for (int k = 0; k < kmax; k += 4) {
-        const cd a0 = Qs[(m0 + g) * C::QSTR + k + t];
-        const cd a1 = Qs[(m0 + g + 8) * C::QSTR + k + t];
+      for (int h = 0; h < 2; ++h)
 #pragma unroll
-        for (int nt = 0; nt < C::NT8; ++nt) {
-          const cd b = Vs[(k + t) * C::VSTR + c0 + nt * 8 + g];
-          double* R = cr[nt];
-          double* I = ci[nt];
-          fdmma(R[0], R[1], R[2], R[3], a0.x, a1.x, b.x);
-          fdmma(R[0], R[1], R[2], R[3], -a0.y, -a1.y, b.y);
-          fdmma(I[0], I[1], I[2], I[3], a0.x, a1.x, b.y);
-          fdmma(I[0], I[1], I[2], I[3], a0.y, a1.y, b.x);
-        }
+        for (int j = 0; j < GW; ++j) acc[i][h][j] = cd{0.0, 0.0};
+    // two k steps a turn, each one's fragments loaded before the other's MMAs; steps past
+    // the beams meet zero entries
+    cd af[2][TW][2], bf[2][GW];
+    auto load = [&](int ks, cd (&x)[TW][2], cd (&y)[GW]) {
+      const uint2 code = codes[ks * kThreads + tid];
+#pragma unroll
+      for (int i = 0; i < TW; ++i)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) x[i][h] = Qs[(row0 + 16 * i + 8 * h) * STR + 4 * ks + t4];
+#pragma unroll
+      for (int j = 0; j < GW; ++j) {
+        const unsigned w = j < 2 ? code.x : code.y, cj = (j & 1) ? w >> 16 : w & 0xffffu;
+        const cd b = tc[cj & 0x7fffu];
+        const double im = __hiloint2double(__double2hiint(b.y) ^ (int)((cj & 0x8000u) << 16),
+                                           __double2loint(b.y));
+        y[j] = (gq & 1) ? cd{im, b.x} : cd{b.x, im};
       }
+    };
+    auto mma = [&](const cd (&x)[TW][2], const cd (&y)[GW]) {
+#pragma unroll
+      for (int j = 0; j < GW; ++j)
+#pragma unroll
+        for (int i = 0; i < TW; ++i)
+          fmma(acc[i][0][j], acc[i][1][j], x[i][0].x, x[i][1].x, y[j].x);
+#pragma unroll
+      for (int j = 0; j < GW; ++j)
+#pragma unroll
+        for (int i = 0; i < TW; ++i)
+          fmma(acc[i][0][j], acc[i][1][j], x[i][0].y, x[i][1].y, y[j].y);
+    };
+    load(0, af[0], bf[0]);
+#pragma unroll 1
+    for (int ks = 0; ks < ng; ks += 2) {
+      load(ks + 1, af[1], bf[1]);
+      mma(af[0], bf[0]);
+      load(min(ks + 2, C::KS - 1), af[0], bf[0]);
+      mma(af[1], bf[1]);
     }
-    __syncthreads();  // every read of Q and V done
-    if (active) {
+    if (C::QB == 1 || nbuf == 1) __syncthreads();  // every read of Q and the column done
+    if (nbuf == 1) fetch();
 #pragma unroll
-      for (int nt = 0; nt < C::NT8; ++nt)
+    for (int i = 0; i < TW; ++i)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int i = m0 + g + ((e >= 2) ? 8 : 0);
-          const int j = c0 + nt * 8 + 2 * t + (e & 1);
-          if (i < n && j < n) {
-            const cd q = Qs[i * C::QSTR + j];
-            const cd acc = cd{cr[nt][e], ci[nt][e]} + q * dreg[nt][e & 1];
-            const cd p = Ps[i * C::PSTR + j] + cb * acc;
-            Ps[i * C::PSTR + j] = p;
-            Qs[i * C::QSTR + j] = q + ca * p;
-          }
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int j = 0; j < GW; ++j) {
+          const int o = (row0 + 16 * i + 8 * h) * STR + col(j);
+          const cd q = Qs[o], z = acc[i][h][j];  // z = -Q V
+          cd p = P(i, h, j);
+          p = cd{fma(cb, fma(q.x, dreg[j], -z.x), p.x), fma(cb, fma(q.y, dreg[j], -z.y), p.y)};
+          P(i, h, j) = p;
+          Qo[o] = cd{fma(ca, p.x, q.x), fma(ca, p.y, q.y)};
         }
+    if (C::QB == 2) {
+      cd* const tmp = Qs;
+      Qs = Qo;
+      Qo = tmp;
     }
   };
   // Gershgorin estimate of Q (cond_est) > 1e3
   auto needs_renorm = [&]() -> bool {
+    constexpr int parts = kThreads / NP;
+    const int j = tid % NP, part = tid / NP;
+    __syncthreads();
+    double t = 0.0;
+    if (part < parts && j < n)
+      for (int i = part; i < n; i += parts)
+        if (i != j) {
+          const cd v = Qs[i * STR + j];
+          t += sqrt(v.x * v.x + v.y * v.y);
+        }
+    csum[tid] = t;
+    __syncthreads();
     double mn = INFINITY, mx = 0.0;
     if (tid < n) {
-      const int j = tid;
-      double tsum = 0.0;
-      for (int i = 0; i < n; ++i)
-        if (i != j) {
-          const cd v = Qs[i * C::QSTR + j];
-          tsum = tsum + sqrt(v.x * v.x + v.y * v.y);
-        }
-      const cd dj = Qs[j * C::QSTR + j];
+      for (int q = 1; q < parts; ++q) t += csum[q * NP + tid];
+      const cd dj = Qs[tid * STR + tid];
       const double ad = hypot(dj.x, dj.y);
-      mn = ad - tsum;
-      mx = ad + tsum;
+      mn = ad - t;
+      mx = ad + t;
     }
     for (int o = 16; o > 0; o >>= 1) {
-      mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-      mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+      mn = fmin(mn, __shfl_xor_sync(full, mn, o));
+      mx = fmax(mx, __shfl_xor_sync(full, mx, o));
     }
     if (lane == 0) {
       red_d[0][warp] = mn;
@@ -215,7 +312,7 @@ __global__ void __launch_bounds__(Cfg<NP>::THREADS)
     }
     __syncthreads();
     if (tid == 0) {
-      for (int w = 1; w < C::WARPS; ++w) {
+      for (int w = 1; w < 4; ++w) {
         mn = fmin(mn, red_d[0][w]);
         mx = fmax(mx, red_d[1][w]);
       }
@@ -229,122 +326,231 @@ __global__ void __launch_bounds__(Cfg<NP>::THREADS)
   };
   // [Q | P] -> [I | Q^{-1} P]
   auto gauss_jordan = [&]() {
-    for (int c = 0; c < n; ++c) {
-      if (warp == 0) {
-        double best = -1.0;
-        int bi = n;
-        for (int r = c + lane; r < n; r += 32) {
-          const double v = cabs1(Qs[r * C::QSTR + c]);
-          if (v > best) {
-            best = v;
-            bi = r;
-          }
-        }
-        for (int o = 16; o > 0; o >>= 1) {
-          const double ov = __shfl_xor_sync(0xffffffffu, best, o);
-          const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-          if (ov > best || (ov == best && oi < bi)) {
-            best = ov;
-            bi = oi;
-          }
-        }
-        if (lane == 0) {
-          piv_sh = bi;
-          if (!(best > 0.0)) atomicOr(a.status, kStatusZeroPivot);
-        }
-      }
-      __syncthreads();
-      const int piv = piv_sh;
-      if (piv != c)
-        for (int j = tid; j < 2 * n; j += C::THREADS) {
-          if (j < n) {
-            if (j >= c) {
-              const cd x = Qs[c * C::QSTR + j];
-              Qs[c * C::QSTR + j] = Qs[piv * C::QSTR + j];
-              Qs[piv * C::QSTR + j] = x;
+    for (int e = tid; e < NP; e += kThreads) slot[e] = -1;
+    if (tid < 64) keys[tid >> 5][tid & 31] = 0;
+    unsigned used = 0;  // rows warp * 16 + gq (+ 8) of the panel: pivots before, or past n
+    const int prow = warp * 16 + gq;
+    if (prow >= n) used |= 1u;
+    if (prow + 8 >= n) used |= 2u;
+    __syncthreads();
+    for (int t = 0; 16 * t < n; ++t) {
+      const int cols = min(16, n - 16 * t);
+      cd x[2][4];
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          x[h][q] = warp < RT ? Qs[(prow + 8 * h) * STR + 16 * t + 4 * q + t4] : cd{0.0, 0.0};
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+#pragma unroll 1
+        for (int tj = 0; tj < 4; ++tj) {
+          const int jj = 4 * q + tj, kb = jj & 1;
+          if (jj >= cols) break;
+          unsigned key = 0;  // see renorm.cu
+          if (t4 == tj) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const unsigned hi = (unsigned)__double2hiint(cabs1(x[h][q]));
+              const unsigned k = ((hi << 1) & ~1023u) | (unsigned)(1023 - (prow + 8 * h));
+              if (!((used >> h) & 1u)) key = max(key, k);
             }
-          } else {
-            const int jp = j - n;
-            const cd x = Ps[c * C::PSTR + jp];
-            Ps[c * C::PSTR + jp] = Ps[piv * C::PSTR + jp];
-            Ps[piv * C::PSTR + jp] = x;
           }
-        }
-      __syncthreads();
-      const cd inv = cdiv(cd{1.0, 0.0}, Qs[c * C::QSTR + c]);
-      const int wq = n - c - 1, W = wq + n;
-      for (int e = tid; e < n * W; e += C::THREADS) {
-        const int r = e / W, jj = e - r * W;
-        if (r == c) continue;
-        const cd f = Qs[r * C::QSTR + c] * inv;
-        if (jj < wq) {
-          const int j = c + 1 + jj;
-          Qs[r * C::QSTR + j] = Qs[r * C::QSTR + j] - f * Qs[c * C::QSTR + j];
-        } else {
-          const int j = jj - wq;
-          Ps[r * C::PSTR + j] = Ps[r * C::PSTR + j] - f * Ps[c * C::PSTR + j];
+          key = __reduce_max_sync(full, key);
+          if (lane == 0) keys[kb][warp] = key;
+          __syncthreads();
+          const int p = 1023 - (int)(max(max(keys[kb][0], keys[kb][1]),
+                                         max(keys[kb][2], keys[kb][3])) & 1023u);
+          const bool holder = warp == (p >> 4) && gq == (p & 7);
+          const int ph = (p >> 3) & 1;
+          if (holder) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+              if (h == ph) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) urow[kb][k * 4 + t4] = x[h][k];
+                used |= 1u << h;
+                if (t4 == tj) {
+                  piv[16 * t + jj] = p;
+                  order[p] = 16 * t + jj;
+                  slot[p] = (signed char)jj;
+                  if (x[h][q].x == 0.0 && x[h][q].y == 0.0) atomicOr(a.status, kStatusZeroPivot);
+                }
+              }
+          }
+          __syncthreads();
+          const cd d = urow[kb][jj];
+          cd u[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) u[k] = urow[kb][k * 4 + t4];
+          const double dinv = 1.0 / (d.x * d.x + d.y * d.y);  // 1/d = conj(d) / |d|^2
+          const cd rc = cd{d.x * dinv, -d.y * dinv};
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const cd f = cd{__shfl_sync(full, x[h][q].x, tj, 4),
+                            __shfl_sync(full, x[h][q].y, tj, 4)} * rc;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) x[h][k] = cfms(f, u[k], x[h][k]);
+            if (t4 == tj) x[h][q] = -f;
+          }
+          if (holder) {  // the pivot row is scaled instead
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+              if (h == ph) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) x[h][k] = u[k] * rc;
+                if (t4 == tj) x[h][q] = rc;
+              }
+          }
+          __syncwarp();
         }
       }
-      __syncthreads();
-      for (int j = tid; j < W; j += C::THREADS) {
-        if (j < wq)
-          Qs[c * C::QSTR + c + 1 + j] = Qs[c * C::QSTR + c + 1 + j] * inv;
-        else
-          Ps[c * C::PSTR + j - wq] = Ps[c * C::PSTR + j - wq] * inv;
+      if (warp < RT) {  // E, in the panel's columns
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int q = 0; q < 4; ++q) Qs[(prow + 8 * h) * STR + 16 * t + 4 * q + t4] = x[h][q];
       }
       __syncthreads();
+      // the other columns: Q's right of the panel, then P's; 16 t + 16 .. of Q first
+#pragma unroll 1
+      for (int pass = 0; pass < 2; ++pass) {
+        const int jmin = pass == 0 ? 16 * t + 16 : 0;  // first column
+        if (jmin >= n) continue;
+#pragma unroll
+        for (int i = 0; i < TW; ++i)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int r = row0 + 16 * i + 8 * h, m = slot[r];
+            if (m >= 0) {
+#pragma unroll
+              for (int j = 0; j < GW; ++j)
+                if (4 * (j * C::WC + wc) >= jmin) {
+                  cd& v = pass == 0 ? Qs[r * STR + col(j)] : P(i, h, j);
+                  c1s[m * STR + col(j)] = v;
+                  v = cd{0.0, 0.0};
+                }
+            }
+          }
+        if (cols < 16)
+          for (int e = tid; e < (16 - cols) * STR; e += kThreads)
+            c1s[cols * STR + e] = cd{0.0, 0.0};
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < GW; ++j) {
+          const int cg = j * C::WC + wc;
+          if (4 * cg < jmin || cg >= ng) continue;
+          cd v[TW][2];
+#pragma unroll
+          for (int i = 0; i < TW; ++i)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+              v[i][h] = pass == 0 ? Qs[(row0 + 16 * i + 8 * h) * STR + col(j)] : P(i, h, j);
+#pragma unroll
+          for (int m0 = 0; m0 < 4; ++m0) {
+            const cd b = c1s[(4 * m0 + t4) * STR + 4 * cg + (gq >> 1)];
+            const double be = (gq & 1) ? b.y : b.x, bo = (gq & 1) ? b.x : -b.y;
+#pragma unroll
+            for (int i = 0; i < TW; ++i) {
+              const cd e0 = Qs[(row0 + 16 * i) * STR + 16 * t + 4 * m0 + t4];
+              const cd e1 = Qs[(row0 + 16 * i + 8) * STR + 16 * t + 4 * m0 + t4];
+              fmma(v[i][0], v[i][1], e0.x, e1.x, be);
+              fmma(v[i][0], v[i][1], e0.y, e1.y, bo);
+            }
+          }
+#pragma unroll
+          for (int i = 0; i < TW; ++i)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              if (pass == 0) Qs[(row0 + 16 * i + 8 * h) * STR + col(j)] = v[i][h];
+              else P(i, h, j) = v[i][h];
+            }
+        }
+        __syncthreads();  // the pivot rows' buffer, Q's next panel
+      }
+      if (tid < cols) slot[piv[16 * t + tid]] = -1;
+      __syncthreads();
     }
-    for (int e = tid; e < n * n; e += C::THREADS) {
-      const int i = e / n, j = e % n;
-      Qs[i * C::QSTR + j] = cd{(i == j) ? 1.0 : 0.0, 0.0};
-    }
+    // P's rows into pivot order, through Q's buffer; Q = I
+#pragma unroll
+    for (int i = 0; i < TW; ++i)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int r = row0 + 16 * i + 8 * h;
+        if (r < n) {
+#pragma unroll
+          for (int j = 0; j < GW; ++j) Qs[order[r] * STR + col(j)] = P(i, h, j);
+        }
+      }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < TW; ++i)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int r = row0 + 16 * i + 8 * h;
+#pragma unroll
+        for (int j = 0; j < GW; ++j) {
+          const int o = r * STR + col(j);
+          if (r < n) P(i, h, j) = Qs[o];
+          Qs[o] = cd{r < n && r == col(j) ? 1.0 : 0.0, 0.0};
+        }
+      }
   };
 
-  const int s = L.s, ns = a.ns;
-  const double dz = a.dz;
-  load_col(0);
-  store_col();
-  __syncthreads();
-  load_col(1);
-  identity_stage(L.bab[0] * dz, L.bab[1] * dz);
-  __syncthreads();
-  store_col();
-  __syncthreads();
   for (int l = 1; l <= ns; ++l) {
-    for (int k = (l == 1) ? 2 : 1; k <= s; ++k) {
-      const int col = s * (l - 1) + k - 1;
-      const double ca = L.bab[2 * k - 1] * dz;
+    for (int k = 1; k <= s; ++k) {
       // k == 1 merges the end-of-slice half kick of slice l-1 with the first kick
-      const double cb = (k == 1) ? 2.0 * L.bab[0] * dz : L.bab[2 * k - 2] * dz;
-      load_col(col + 1);  // the next stage's matrix (the last column after slice ns)
-      product_stage(cb, ca);
-      store_col();        // V is no longer read: the next stage's matrix goes in
-      __syncthreads();
+      const double cb = (k == 1) ? (l == 1 ? 1.0 : 2.0) * L.bab[0] * dz : L.bab[2 * k - 2] * dz;
+      stage(cb, L.bab[2 * k - 1] * dz);
     }
     const bool last = l == ns;
     bool renorm = last;
     if (!last) renorm = (L.policy == 0) ? needs_renorm() : (l % a.interval) == 0;
     if (renorm) {
-      gauss_jordan();
       __syncthreads();
+      gauss_jordan();
     }
   }
   // final half kick with Q = I: P += b1 dz M(end)
-  identity_stage(L.bab[0] * dz, 0.0);
+  stage(L.bab[0] * dz, 0.0);
+  if (tid == 0 && dead)  // copies still on their way (as long as they may take)
+    while (consumed < issued) {
+      wait_parity(&bars[out], parity);
+      ++consumed;
+      if (++out == nbuf) {
+        out = 0;
+        parity ^= 1;
+      }
+    }
   __syncthreads();
-  for (int e = tid; e < n * n; e += C::THREADS) {
+  for (int e = tid; e < n * n; e += kThreads) {
     const int i = e / n, j = e % n;
-    Qg[(size_t)i * ld + j] = Qs[i * C::QSTR + j];
-    Pg[(size_t)i * ld + j] = Ps[i * C::PSTR + j];
+    Qg[(size_t)i * ld + j] = Qs[i * STR + j];
   }
+#pragma unroll
+  for (int i = 0; i < TW; ++i)
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int j = 0; j < GW; ++j) {
+        const int r = row0 + 16 * i + 8 * h;
+        if (r < n && col(j) < n) Pg[(size_t)r * ld + col(j)] = P(i, h, j);
+      }
 }
 
-template <int NP>
-void launch(const FusedLaunch& L, cudaStream_t st) {
-  using C = Cfg<NP>;
+template <int RT, int GW>
+void launch(const FusedLaunch& L, int nvmax, cudaStream_t st) {
+  using C = Cfg<RT, GW>;
   static SmemOptIn attr;
-  attr.ensure((const void*)k_fused_rkn<NP>, C::SMEM);
-  k_fused_rkn<NP><<<L.total_ctas, C::THREADS, C::SMEM, st>>>(L);
+  const int stride = 2 * (nvmax + 1);
+  // four column buffers where they leave the CTAs per SM the registers allow, else one or
+  // two (a column's copy takes longer than a stage of a small problem)
+  auto bytes = [&](int b) { return (C::elems + (size_t)b * stride) * sizeof(cd); };
+  int nbuf = bytes(kTabBufs) <= size_t(227 * 1024) / C::MINB - 4096 ? kTabBufs : 2;
+  if (bytes(nbuf) > 224 * 1024) nbuf = 1;
+  const size_t smem = (C::elems + (size_t)nbuf * stride) * sizeof(cd);
+  attr.ensure((const void*)k_fused_rkn<RT, GW>, smem);
+  k_fused_rkn<RT, GW><<<L.total_ctas, kThreads, smem, st>>>(L, nbuf, stride);
 }
 
 }  // namespace fused
@@ -352,24 +558,27 @@ void launch(const FusedLaunch& L, cudaStream_t st) {
 int launch_fused_rkn(const FusedLaunch& L, cudaStream_t st) {
   if (L.nprob < 1 || L.nprob > kFusedMaxProblems || L.s < 1 || L.s > 11)
     throw std::invalid_argument("fused integration: bad launch");
-  int nmax = 0, ctas = 0;
+  int nmax = 0, nvmax = 0, ctas = 0;
   for (int q = 0; q < L.nprob; ++q) {
     const FusedProblem& a = L.p[q];
     if (a.n < 2 || a.n > kFusedMaxBeams || a.ns < 1 || a.interval < 1 || a.nang < 1 ||
-        a.first_cta != ctas)
+        a.first_cta != ctas || a.nv < 1 || a.nv > kFusedMaxEntries)
       throw std::invalid_argument("fused integration: unsupported problem");
     ctas += a.nang;
     nmax = std::max(nmax, a.n);
+    nvmax = std::max(nvmax, a.nv);
   }
   if (ctas != L.total_ctas) throw std::invalid_argument("fused integration: CTA count");
   if (nmax <= 16)
-    fused::launch<16>(L, st);
+    fused::launch<1, 1>(L, nvmax, st);
+  else if (nmax <= 24)
+    fused::launch<2, 3>(L, nvmax, st);
   else if (nmax <= 32)
-    fused::launch<32>(L, st);
+    fused::launch<2, 4>(L, nvmax, st);
   else if (nmax <= 48)
-    fused::launch<48>(L, st);
+    fused::launch<3, 3>(L, nvmax, st);
   else
-    fused::launch<64>(L, st);
+    fused::launch<4, 4>(L, nvmax, st);
   return 1;
 }
 

@@ -8,9 +8,11 @@
 
 namespace trhepd {
 
-// Largest beam count of the fused kernel: Q, P and the stage matrix of one angle
-// (64 x 64 complex each, padded rows) fill 202 KB of shared memory.
+// Largest beam count of the fused kernel: Q, P, the pivot rows and one table column of an
+// angle (64 x 68 complex each of the first two) fit the 227 KB of shared memory.
 constexpr int kFusedMaxBeams = 64;
+// Table entries per stage column it takes: every beam difference of 64 beams and more.
+constexpr int kFusedMaxEntries = 2100;
 
 // One problem of a fused launch: its RKN integration (hp_int_spa,
 // surf_prkn.f90:278-330).  Q and P enter as the state after invstransh (Q = I)

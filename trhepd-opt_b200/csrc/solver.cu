@@ -765,7 +765,8 @@ void run_rkn(trhepd_context* C, trhepd_problem& Pb, int precision, RunState& R) 
   const double dz = Pb.dz;
   begin_run(C, Pb, precision, I.s * Pb.ns, R, context_workspace(C));
   const bool every_slice = (Pb.n == 1 && Pb.int_method == 6);  // hp_int_spa1d renormalises each slice
-  if (!R.split && R.nprob == 1 && Pb.n >= 2 && Pb.n <= std::min(C->fused_max_n, kFusedMaxBeams)) {
+  if (!R.split && R.nprob == 1 && Pb.n >= 2 && Pb.n <= std::min(C->fused_max_n, kFusedMaxBeams) &&
+      Pb.nv <= kFusedMaxEntries) {
     // whole integration in one launch, state in shared memory (small.cu)
     static thread_local FusedLaunch L;  // 17 KB of kernel parameters
     L.nprob = 1;
@@ -1199,7 +1200,7 @@ void batch_solve(trhepd_context* C, trhepd_problem* const* probs, int count, int
   for (int q = 0; q < count; ++q) {
     trhepd_problem* p = probs[q];
     if (!p) throw std::invalid_argument("null problem in batch");
-    if (p->I.family == kRkn && p->n >= 2 && p->n <= fmax)
+    if (p->I.family == kRkn && p->n >= 2 && p->n <= fmax && p->nv <= kFusedMaxEntries)
       fused[p->I.s == 6 ? 0 : 1].push_back(p);
     else
       rest.push_back(p);
