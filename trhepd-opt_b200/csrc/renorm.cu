@@ -71,6 +71,20 @@ __device__ __forceinline__ void mma64(double& c0, double& c1, double& c2, double
       : "d"(a0), "d"(a1), "d"(b0));
 }
 
+__device__ __forceinline__ void cp16(void* smem, const void* gmem, bool pred) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(gmem),
+               "r"(pred ? 16 : 0));
+}
+// 1 / d by two Newton-Raphson steps y <- y + y (1 - d y) on the hardware's approximation
+// (about 2^-22): within an ulp or two, at a quarter of the division's latency.
+__device__ __forceinline__ double reciprocal(double d) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+  y = fma(y, fma(-d, y, 1.0), y);
+  return fma(y, fma(-d, y, 1.0), y);
+}
+
 // One cluster of `ctas` CTAs per angle.  kG = 1: CTA s holds the block's columns 16 s ..;
 // kG = 2 (the whole of [Q | P], c0 = 0, w = n): also P's columns 16 s .., and the
 // elimination is finished here (permuted P, Q = I).
@@ -83,18 +97,19 @@ __device__ __forceinline__ void mma64(double& c0, double& c1, double& c2, double
 // (re, im) column pairs, K ordered so that lane t's A values of two k-steps are the
 // parts of one complex E entry.
 //
-// The step chain (key, two reductions, pivot row, reciprocal, update) bounds a
-// sub-panel.  The reductions are one redux.sync each on a 32-bit key: the exponent and
-// 11 leading mantissa bits of |re|+|im| over the row number, so the pivot is the largest
-// to within 2^-11 (the lowest such row), which bounds the multipliers by 1.0005 instead
-// of 1.
+// The step chain (key, reduction, candidate rows, barrier, reciprocal, update; 1.1 K
+// clocks at n = 47, 2.6 K at n = 521) bounds a sub-panel.  One redux.sync on a 32-bit key:
+// the exponent and 11 leading mantissa bits of |re|+|im| over the row number, so the
+// pivot is the largest to within 2^-11, which bounds the multipliers by 1.0005 instead of
+// 1.  The column group at hand is always x[.][0], the groups rotate: one copy of the step
+// in the instruction stream for the taller warps.
 template <int kG, int kRT, int kMaxT, int kMinB>
 __global__ void __launch_bounds__(kMaxT, kMinB) k_gj_block(const BlockArgs g, int ctas) {
   const int a = blockIdx.x / ctas, s = blockIdx.x - a * ctas;
   if (g.flag && !g.flag[a]) return;  // the whole cluster
   constexpr int kWarps = kMaxT / 32, kCStr = kW * kG + 4, kR = 2 * kRT, kWarpRows = 16 * kRT;
-  __shared__ unsigned keys[2][32];
-  __shared__ cd urow[2][kW];
+  __shared__ __align__(16) unsigned keys[2][32];
+  __shared__ cd urow[2][kWarps][kW];
   __shared__ cd c1s[kW][kCStr];
   __shared__ int pivs[kW];
   __shared__ signed char slot[kWarps * kWarpRows];  // row -> pivot step of the E being applied
@@ -129,7 +144,7 @@ __global__ void __launch_bounds__(kMaxT, kMinB) k_gj_block(const BlockArgs g, in
   for (int t = 0; t < g.nsub; ++t) {
     const int cbase = g.c0 + t * kW;
     if (s == t) {
-#pragma unroll
+#pragma unroll (kRT == 1 ? 4 : 1)
       for (int q = 0; q < 4; ++q) {
 #pragma unroll 1
         for (int tj = 0; tj < 4; ++tj) {
@@ -140,59 +155,77 @@ __global__ void __launch_bounds__(kMaxT, kMinB) k_gj_block(const BlockArgs g, in
           if (t4 == tj) {
 #pragma unroll
             for (int r = 0; r < kR; ++r) {
-              const unsigned hi = (unsigned)__double2hiint(cabs1(x[r][q]));
+              const unsigned hi = (unsigned)__double2hiint(cabs1(x[r][0]));
               const unsigned k = ((hi << 1) & ~1023u) | (unsigned)(1023 - (row0 + 8 * r));
               if (!((used >> r) & 1u)) key = max(key, k);
             }
           }
           key = __reduce_max_sync(full, key);
           if (lane == 0) keys[buf][warp] = key;
+          // every warp publishes its candidate row before the one barrier
+          const int own = 1023 - (int)(key & 1023u) - warp * kWarpRows;
+          const int cr = key != 0 && gq == (own & 7) ? own >> 3 : -1;
+#pragma unroll
+          for (int r = 0; r < kR; ++r)
+            if (r == cr) {
+#pragma unroll
+              for (int k = 0; k < 4; ++k) urow[buf][warp][((q + k) & 3) * 4 + t4] = x[r][k];
+            }
           __syncthreads();
-          const int p = 1023 - (int)(__reduce_max_sync(full, keys[buf][lane]) & 1023u);
-          const int pl = p - warp * kWarpRows;  // the pivot row within this warp's
-          const bool holder = pl >= 0 && pl < kWarpRows && gq == (pl & 7);
-          const int pr = pl >> 3;
-          if (holder) {
+          unsigned top = 0;
 #pragma unroll
-            for (int r = 0; r < kR; ++r)
-              if (r == pr) {
-#pragma unroll
-                for (int k = 0; k < 4; ++k) urow[buf][k * 4 + t4] = x[r][k];
-                used |= 1u << r;
-                if (t4 == tj) {
-                  piv[cbase + jj] = p;
-                  order[p] = cbase + jj;
-                  if (x[r][q].x == 0.0 && x[r][q].y == 0.0) atomicOr(g.status, kStatusZeroPivot);
-                }
-              }
+          for (int w = 0; w < kWarps; w += 4) {
+            const uint4 v = *reinterpret_cast<const uint4*>(&keys[buf][w]);
+            top = max(max(max(top, v.x), max(v.y, v.z)), v.w);
           }
-          __syncthreads();
-          const cd d = urow[buf][jj];
+          const int p = 1023 - (int)(top & 1023u);
+          const int pw = p / kWarpRows, pl = p - warp * kWarpRows;  // its warp; within this one
+          const cd* up = urow[buf][pw];
+          const cd d = up[jj];
           cd u[4];
 #pragma unroll
-          for (int k = 0; k < 4; ++k) u[k] = urow[buf][k * 4 + t4];
-          const double dinv = 1.0 / (d.x * d.x + d.y * d.y);  // 1/d = conj(d) / |d|^2
+          for (int k = 0; k < 4; ++k) u[k] = up[((q + k) & 3) * 4 + t4];
+          const double dinv = reciprocal(fma(d.x, d.x, d.y * d.y));  // 1/d = conj(d) / |d|^2
           const cd rc = cd{d.x * dinv, -d.y * dinv};
 #pragma unroll
           for (int r = 0; r < kR; ++r) {
             // the row's entry of column jj is lane (gq, tj)'s
-            const cd f = cd{__shfl_sync(full, x[r][q].x, tj, 4),
-                            __shfl_sync(full, x[r][q].y, tj, 4)} * rc;
+            const cd f = cd{__shfl_sync(full, x[r][0].x, tj, 4),
+                            __shfl_sync(full, x[r][0].y, tj, 4)} * rc;
 #pragma unroll
             for (int k = 0; k < 4; ++k) x[r][k] = cfms(f, u[k], x[r][k]);
-            if (t4 == tj) x[r][q] = -f;
+            if (t4 == tj) x[r][0] = -f;
           }
-          if (holder) {  // the pivot row is scaled instead
+          if (pl >= 0 && pl < kWarpRows && gq == (pl & 7)) {  // the pivot row is scaled instead
+            const int pr = pl >> 3;
+            used |= 1u << pr;
 #pragma unroll
             for (int r = 0; r < kR; ++r)
               if (r == pr) {
 #pragma unroll
                 for (int k = 0; k < 4; ++k) x[r][k] = u[k] * rc;
-                if (t4 == tj) x[r][q] = rc;
+                if (t4 == tj) x[r][0] = rc;
               }
+            if (t4 == tj) {
+              pivs[jj] = p;
+              if (d.x == 0.0 && d.y == 0.0) atomicOr(g.status, kStatusZeroPivot);
+            }
           }
           __syncwarp();
         }
+#pragma unroll
+        for (int r = 0; r < kR; ++r) {
+          const cd f = x[r][0];
+#pragma unroll
+          for (int k = 1; k < 4; ++k) x[r][k - 1] = x[r][k];
+          x[r][3] = f;
+        }
+      }
+      // the pivots leave in one go: a global store per step would hold up its barrier
+      __syncthreads();
+      if (tid < cols) {
+        piv[cbase + tid] = pivs[tid];
+        order[pivs[tid]] = cbase + tid;
       }
 #pragma unroll
       for (int r = 0; r < kR; ++r)
@@ -273,61 +306,71 @@ __global__ void __launch_bounds__(kMaxT, kMinB) k_gj_block(const BlockArgs g, in
 // C1_u.  (Folding the sub-panels' E into one E of the block instead would need no such
 // chain, but its entries grow with the block: 8e-11 instead of 2e-11 of the row maximum
 // on the reference's N = 521 case at 0.68 A with sp6.)
-constexpr int kC1Cols = 32, kC1Str = kC1Cols + 4;
+// The rows and the E they take (nsub (nsub - 1) / 2 blocks of 16 x 16) are all copied into
+// shared memory first: one memory latency instead of one per few k steps.
+constexpr int kC1Cols = 32, kC1Str = kC1Cols + 4, kEStr = 20;
+static size_t c1_bytes(int nsub) {
+  return ((size_t)nsub * kW * kC1Str + (size_t)nsub * (nsub - 1) / 2 * kW * kEStr) * sizeof(cd);
+}
 __global__ void __launch_bounds__(128) k_gj_c1(const BlockArgs g) {
   const int a = blockIdx.y;
   if (g.flag && !g.flag[a]) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  cd* c1 = reinterpret_cast<cd*>(smem_raw);  // 16 nsub x kC1Str
-  __shared__ int prow[kMaxBlock * kW];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, gq = lane >> 2, t4 = lane & 3;
   const int n = g.n, rows = g.nsub * kW, vc0 = blockIdx.x * kC1Cols;
+  cd* c1 = reinterpret_cast<cd*>(smem_raw);  // 16 nsub x kC1Str
+  cd* es = c1 + rows * kC1Str;               // block (t, u < t): t (t - 1) / 2 + u, 16 x kEStr
   const int n0 = n - g.c0 - g.w, total = n0 + n;
   const cd* E = g.E + (size_t)a * n * g.ew;
   const cd* Qa = g.Q + (size_t)a * n * g.ld + g.c0 + g.w;
   const cd* Pa = g.P + (size_t)a * n * g.ld;
-  if (tid < rows) prow[tid] = tid < g.w ? g.piv[(size_t)a * n + g.c0 + tid] : -1;
-  __syncthreads();
+  const int* piv = g.piv + (size_t)a * n + g.c0;
   {
     const int vc = vc0 + lane;
     const cd* src = vc < n0 ? Qa + vc : Pa + (vc - n0);
-#pragma unroll 8
+#pragma unroll 4
     for (int m = warp; m < rows; m += 4) {
-      const int pr = prow[m];
-      c1[m * kC1Str + lane] =
-          (pr >= 0 && vc < total) ? src[(size_t)pr * g.ld] : cd{0.0, 0.0};
+      const bool ok = m < g.w && vc < total;
+      cp16(c1 + m * kC1Str + lane, ok ? src + (size_t)piv[m] * g.ld : g.Q, ok);
     }
+    for (int t = 1; t < g.nsub; ++t)
+#pragma unroll 4
+      for (int e = tid; e < t * kW * kW; e += 128) {
+        const int u = e / (kW * kW), r = (e / kW) % kW, k = e % kW, m = t * kW + r;
+        const bool ok = m < g.w;  // a missing pivot row's result is unused
+        cp16(es + ((size_t)(t * (t - 1) / 2 + u) * kW + r) * kEStr + k,
+             ok ? E + (size_t)piv[m] * g.ew + u * kW + k : E, ok);
+      }
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
   }
   __syncthreads();
   const int cw = warp * 8;  // this warp's columns
   for (int t = 1; t < g.nsub; ++t) {
     cd acc[2][2];  // [row half][4-column group]
-    const cd* er[2];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int m = t * kW + gq + 8 * h;
-      er[h] = E + (size_t)max(prow[m], 0) * g.ew + t4;  // a missing pivot row's result is unused
+    for (int h = 0; h < 2; ++h)
 #pragma unroll
-      for (int q = 0; q < 2; ++q) acc[h][q] = c1[m * kC1Str + cw + q * 4 + t4];
-    }
-#pragma unroll 4
-    for (int k = 0; k < t * kW; k += 4) {
-      const cd e0 = er[0][k], e1 = er[1][k];
+      for (int q = 0; q < 2; ++q)
+        acc[h][q] = c1[(t * kW + gq + 8 * h) * kC1Str + cw + q * 4 + t4];
+    for (int u = 0; u < t; ++u) {
+      const cd* eb = es + ((size_t)(t * (t - 1) / 2 + u) * kW + gq) * kEStr + t4;
 #pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        const cd b = c1[(k + t4) * kC1Str + cw + q * 4 + (gq >> 1)];
-        const double be = (gq & 1) ? b.y : b.x, bo = (gq & 1) ? b.x : -b.y;
-        mma64(acc[0][q].x, acc[0][q].y, acc[1][q].x, acc[1][q].y, e0.x, e1.x, be);
-        mma64(acc[0][q].x, acc[0][q].y, acc[1][q].x, acc[1][q].y, e0.y, e1.y, bo);
+      for (int k = 0; k < kW; k += 4) {
+        const cd e0 = eb[k], e1 = eb[8 * kEStr + k];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const cd b = c1[(u * kW + k + t4) * kC1Str + cw + q * 4 + (gq >> 1)];
+          const double be = (gq & 1) ? b.y : b.x, bo = (gq & 1) ? b.x : -b.y;
+          mma64(acc[0][q].x, acc[0][q].y, acc[1][q].x, acc[1][q].y, e0.x, e1.x, be);
+          mma64(acc[0][q].x, acc[0][q].y, acc[1][q].x, acc[1][q].y, e0.y, e1.y, bo);
+        }
       }
     }
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int m = t * kW + gq + 8 * h;
+    for (int h = 0; h < 2; ++h)
 #pragma unroll
       for (int q = 0; q < 2; ++q)
-        c1[m * kC1Str + cw + q * 4 + t4] = m < g.w ? acc[h][q] : cd{0.0, 0.0};
-    }
+        c1[(t * kW + gq + 8 * h) * kC1Str + cw + q * 4 + t4] = acc[h][q];
     __syncwarp();  // a warp reads only its own columns
   }
   __syncthreads();
@@ -347,11 +390,6 @@ constexpr int ASTR = BK + 4, BSTR = BN + 4;
 constexpr int A_TILE = BM * ASTR, B_TILE = BK * BSTR;
 constexpr size_t UPD_SMEM = (size_t)STAGES * (A_TILE + B_TILE) * sizeof(cd);
 
-__device__ __forceinline__ void cp16(void* smem, const void* gmem, bool pred) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(gmem),
-               "r"(pred ? 16 : 0));
-}
 __global__ void __launch_bounds__(128, 2) k_gj_update(const BlockArgs g) {
   const int a = blockIdx.z;
   if (g.flag && !g.flag[a]) return;
@@ -512,8 +550,8 @@ static bool whole(int n) { return n <= kMaxBlock * kW; }  // one launch
 // clusters fit about one wave, else four.  Whole elimination at n = 521 (one CTA per SM)
 // with 2 / 4 / 6 / 8 sub-panels per block: 1 angle 1.40 / 1.33 / 1.34 / 1.36 ms, 16
 // angles 3.22 / 2.72 / 2.55 / 2.79, 31 angles 4.95 / 4.07 / 4.44 / 4.87, 61 angles 8.28 /
-// 7.73 / 7.93 / 8.47 (rank-32 updates with physical row swaps and a launch per 16
-// columns: 4.2, 5.9, 6.8, 10.7 ms).
+// 7.73 / 7.93 / 8.47 (one barrier per step since: 1.24, 2.53, 4.01, 7.57; rank-32 updates
+// with physical row swaps and a launch per 16 columns took 4.2, 5.9, 6.8, 10.7 ms).
 static int block_ctas(int nang, int n) {
   const int sub = ceil_div(n, kW);
   if (whole(n)) return sub;
@@ -590,7 +628,7 @@ int launch_gj_cluster(cd* Q, cd* P, const int* flag, int nang, int n, int ld, vo
     return 1;
   }
   static SmemOptIn upd, fin, cone;
-  cone.ensure((const void*)k_gj_c1, (size_t)kMaxBlock * kW * kC1Str * sizeof(cd));
+  cone.ensure((const void*)k_gj_c1, c1_bytes(kMaxBlock));
   upd.ensure((const void*)k_gj_update, UPD_SMEM);
   const size_t fin_smem = (size_t)n * kPermCols * sizeof(cd);
   fin.ensure((const void*)k_gj_finish, fin_smem);
@@ -614,8 +652,7 @@ int launch_gj_cluster(cd* Q, cd* P, const int* flag, int nang, int n, int ld, vo
       h.E += (size_t)a0 * n * g.ew;
       h.C1 += (size_t)a0 * g.c1stride;
       const int na = std::min(nang - a0, 65535);
-      k_gj_c1<<<dim3(ceil_div(total, kC1Cols), na), 128, (size_t)g.nsub * kW * kC1Str * sizeof(cd),
-                st>>>(h);
+      k_gj_c1<<<dim3(ceil_div(total, kC1Cols), na), 128, c1_bytes(g.nsub), st>>>(h);
       k_gj_update<<<dim3(ceil_div(total, BN), ceil_div(n, BM), na), 128, UPD_SMEM, st>>>(h);
       launches += 2;
     }
