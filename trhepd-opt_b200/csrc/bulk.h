@@ -22,6 +22,16 @@ struct BatchedGemm {
 };
 void launch_zgemm_batched(const BatchedGemm& g, cudaStream_t st);
 
+// The reflection matrices R (nitem x n x ld) of every item, all slices and layers in one
+// launch (groups of up to 8 beams).  fc, fs: the nine Taylor coefficients 1/(2k)! and
+// 1/(2k+1)!; m double-angle steps on h = dz / 2^m; phase may be null; *layers (zeroed by
+// the caller) receives the most layers of any item.
+bool bulk_small_fits(int n);
+void launch_bulk_small(const TableEntry* table, int nv, int ns, const int* pair, const cd* gam,
+                       const int* gsize, int ngr, int n, int nitem, int m, double h,
+                       const double* fc, const double* fs, const cd* phase, int ml, double epsb,
+                       cd* R, int ld, int* layers, unsigned* status, cudaStream_t st);
+
 // items b = angle * ngr + group, every matrix padded to n x n (ld) / 2n x 2n (ld2)
 void launch_bulk_hamiltonian(const TableEntry* tcol, const int* pair, const cd* gam,
                              const int* gsize, int ngr, int n, int ld, int batch, double h2, cd* H,

@@ -1473,7 +1473,15 @@ void bulk_solve(trhepd_context* C, BulkInputs& B, std::vector<std::vector<cd>>& 
     }
   }
   CK(cudaEventRecord(C->ev0, st));
-  for (int l = 0; l < ns; ++l) {
+  const bool fused = bulk_small_fits(n);
+  unsigned* status = (unsigned*)C->status.ensure(16);
+  CK(cudaMemsetAsync(status, 0, 16, st));
+  cd* R = buf1(15);
+  CK(cudaMemsetAsync(R, 0, nb1 * sizeof(cd), st));
+  if (fused)
+    launch_bulk_small(table, nv, ns, d_pair, d_gam, d_gsize, ngr, n, nitem, m, h, fc, fs,
+                      shifted ? d_ph : nullptr, B.ml, B.epsb, R, ld, (int*)status + 1, status, st);
+  for (int l = 0; l < ns && !fused; ++l) {
     launch_bulk_hamiltonian(table + (size_t)l * nv, d_pair, d_gam, d_gsize, ngr, n, ld, nitem,
                             h * h, H, X, st);
     gemm1(X, X, X2, 0, nullptr);
@@ -1504,20 +1512,16 @@ void bulk_solve(trhepd_context* C, BulkInputs& B, std::vector<std::vector<cd>>& 
     }
   }
   cd* Tm = Et;  // unit-layer transfer matrix
-  if (shifted) launch_bulk_phase_cols(Tm, d_ph, d_gsize, ngr, n, ld2, nitem, st);
+  if (shifted && !fused) launch_bulk_phase_cols(Tm, d_ph, d_gsize, ngr, n, ld2, nitem, st);
   // layer recursion with the convergence exit
   std::vector<int> act(nitem, 1);
   int* d_act = upload(C->bk[13], act, st);
   double* r20 = (double*)C->bk[14].ensure((size_t)nitem * n * sizeof(double));
-  cd* R = buf1(15);
   cd* Qg = buf1(16);
   cd* Pg = buf1(17);
-  unsigned* status = (unsigned*)C->status.ensure(16);
-  CK(cudaMemsetAsync(status, 0, 16, st));
-  CK(cudaMemsetAsync(R, 0, nb1 * sizeof(cd), st));
   void* gjs = C->gj.ensure(gj_scratch_bytes(nitem, n));
   int layers = 0;
-  for (int l = 1; l <= B.ml; ++l) {
+  for (int l = 1; l <= B.ml && !fused; ++l) {
     launch_bulk_layer_init(Tm, d_act, n, ld, ld2, nitem, T1, T2, st);
     if (l > 1) {
       gemm_t(Tm, R, T1, d_act);                       // T12 + T11 R
@@ -1544,6 +1548,7 @@ void bulk_solve(trhepd_context* C, BulkInputs& B, std::vector<std::vector<cd>>& 
   CK(cudaGetLastError());
   float ms = 0;
   cudaEventElapsedTime(&ms, C->ev0, C->ev1);
+  if (fused) layers = (int)hs[1];
   if (hs[0] & kStatusZeroPivot) throw CudaError("zero pivot in the bulk layer solve", TRHEPD_ENONFINITE);
   records.assign(nitem, {});
   for (int b = 0; b < nitem; ++b) {
