@@ -7,10 +7,12 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdint>
 #include <cstdio>
 #include <cstring>
 #include <functional>
 #include <stdexcept>
+#include <unordered_map>
 
 #include "fortran_text.h"
 #include "scattering_tables.h"
@@ -418,19 +420,24 @@ void load_surface_inputs(const std::string& bulkp, const std::string& surf, doub
   // srfghk (surfsub.f90:9-41): beam-difference index of every pair l > k
   S.iv.assign((size_t)S.nb * S.nb, 0);
   {
+    // the reference scans the list for each pair (first match from entry 1 on); the same
+    // answers from a hash of the list
     int nv = S.nvb;
+    std::unordered_map<uint64_t, int> at;
+    at.reserve((size_t)4 * S.nb + nv);
+    auto key = [](int dh, int dk) { return (uint64_t)(uint32_t)dh << 32 | (uint32_t)dk; };
+    for (int m = 1; m < nv; ++m) at.emplace(key(igh[m], igk[m]), m);  // keeps the first
     for (int k = 0; k < S.nb - 1; ++k)
       for (int l = k + 1; l < S.nb; ++l) {
-        int dh = S.ih[l] - S.ih[k], dk = S.ik[l] - S.ik[k], m = 1;
-        for (; m < nv; ++m)
-          if (igh[m] == dh && igk[m] == dk) break;
-        if (m == nv) {
+        const int dh = S.ih[l] - S.ih[k], dk = S.ik[l] - S.ik[k];
+        const auto [it, added] = at.emplace(key(dh, dk), nv);
+        if (added) {
           if (nv + 1 > nvm) throw std::runtime_error("srfghk: nv exceeds beam pairs");
           igh[nv] = dh;
           igk[nv] = dk;
           ++nv;
         }
-        S.iv[(size_t)k * S.nb + l] = m + 1;
+        S.iv[(size_t)k * S.nb + l] = it->second + 1;
       }
     S.nv = nv;
   }

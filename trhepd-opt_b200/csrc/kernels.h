@@ -106,6 +106,11 @@ int launch_gj_cluster(cd* Q, cd* P, const int* flag, int nang, int n, int ld, vo
 // RK4 stage combination (rk4_int, surf_rk.f90:27-91); see kernels_f64.cu.
 void launch_rk4_combine(cd* Q, cd* P, cd* Qt, cd* Pt, cd* KP, cd* SQ, cd* SP, int j, double w,
                         double step, double h6, int nang, int n, int ld, cudaStream_t st);
+// Bulk reflection records into F (nang x n x n, row-major, zeroed by the caller), permuted
+// by iord (surflf.f90:105-115): per angle `per` values, group l's first[l+1] - first[l]
+// beams as a column-major block.
+void launch_scatter_records(const cd* rec, size_t per, const int* first, int ngr, const int* iord,
+                            int nang, int n, cd* F, cudaStream_t st);
 // invstransh (matcomp.f90:140-172): Q = I + F^H, P = I - F^H, from F (nang x n x n, row-major).
 void launch_invstransh_build(const cd* F, cd* Q, cd* P, int nang, int n, int ld, cudaStream_t st);
 // P(i,j) = i * P(i,j) * conj(g_i)  (after the solve)

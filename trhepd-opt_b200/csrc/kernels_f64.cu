@@ -761,6 +761,31 @@ void launch_rk4_combine(cd* Q, cd* P, cd* Qt, cd* Pt, cd* KP, cd* SQ, cd* SP, in
   k_rk4_combine<<<grid, 128, 0, st>>>(Q, P, Qt, Pt, KP, SQ, SP, j, w, step, h6, n, ld);
 }
 
+// ============================================================ bulk records
+// A CTA per (group, angle); F is filled here instead of on the host, which wrote and
+// uploaded all n x n values of every angle (n = 521, 16 angles: 70 MB, of which the four
+// groups' blocks are 17).
+__global__ void k_scatter_records(const cd* __restrict__ rec, size_t per,
+                                  const int* __restrict__ first, const int* __restrict__ iord,
+                                  int nang, int n, cd* __restrict__ F) {
+  const int l = blockIdx.x, b0 = first[l], m = first[l + 1] - b0;
+  size_t off = 0;
+  for (int g = 0; g < l; ++g) off += (size_t)(first[g + 1] - first[g]) * (first[g + 1] - first[g]);
+  for (int t = blockIdx.y; t < nang; t += gridDim.y) {
+    const cd* src = rec + (size_t)t * per + off;
+    cd* dst = F + (size_t)t * n * n;
+    for (int e = threadIdx.x; e < m * m; e += blockDim.x) {
+      const int j = e / m, i = e - j * m;
+      dst[(size_t)(iord[b0 + i] - 1) * n + iord[b0 + j] - 1] = src[e];
+    }
+  }
+}
+void launch_scatter_records(const cd* rec, size_t per, const int* first, int ngr, const int* iord,
+                            int nang, int n, cd* F, cudaStream_t st) {
+  k_scatter_records<<<dim3(ngr, std::min(nang, 65535)), 256, 0, st>>>(rec, per, first, iord, nang,
+                                                                      n, F);
+}
+
 // ============================================================ boundary transforms
 __global__ void k_invstransh_build(const cd* __restrict__ F, cd* __restrict__ Q,
                                    cd* __restrict__ P, int n, int ld) {

@@ -371,7 +371,7 @@ void prepare(trhepd_context* C, const SolveArgs& A, trhepd_problem& Pb) {
   Pb.nang = nang;
   Pb.nrep2 = nrep2;
   Pb.ld = ld;
-  std::vector<cd> gam((size_t)nang * n), Dm((size_t)nang * ld, cd{0, 0}), F((size_t)nang * n * n);
+  std::vector<cd> gam((size_t)nang * n), Dm((size_t)nang * ld, cd{0, 0});
   std::vector<double> wnsga2(nang);
   Pb.angle_deg.assign(nang, 0.0);
   size_t per = 0;
@@ -409,20 +409,6 @@ void prepare(trhepd_context* C, const SolveArgs& A, trhepd_problem& Pb) {
       if (s < 0) kappa_max = std::max(kappa_max, std::sqrt(-s));
     }
     Pb.angle_deg[t] = (ng_outer ? ga : az) * 180.0 / 3.141592654;
-    // bulk f permuted by iord (surflf.f90:105-115); F row-major (i, j)
-    const double* rec = A.t1 + 2 * per * t;
-    cd* Ft = F.data() + (size_t)t * n * n;
-    int ib1 = 0;
-    size_t o = 0;
-    for (int l = 0; l < A.ngr; ++l) {
-      int m = A.nbg[l];
-      for (int j = 0; j < m; ++j)
-        for (int i = 0; i < m; ++i, ++o) {
-          int r = A.iord[ib1 + i] - 1, c = A.iord[ib1 + j] - 1;
-          Ft[(size_t)r * n + c] = cd{rec[2 * o], rec[2 * o + 1]};
-        }
-      ib1 += m;
-    }
   }
   Pb.kappa_max = kappa_max;
   Pb.nb0 = 0;
@@ -430,7 +416,19 @@ void prepare(trhepd_context* C, const SolveArgs& A, trhepd_problem& Pb) {
     if (A.ih[i] == 0 && A.ik[i] == 0) Pb.nb0 = i;
   upload(Pb.gam, gam, st);
   upload(Pb.D, Dm, st);
-  upload(Pb.F, F, st);
+  {  // bulk f permuted by iord (surflf.f90:105-115), scattered on the device
+    std::vector<int> first(A.ngr + 1, 0);
+    for (int l = 0; l < A.ngr; ++l) first[l + 1] = first[l] + A.nbg[l];
+    const std::vector<int> iord(A.iord, A.iord + n);
+    const int* d_first = upload(C->simg, first, st);
+    const int* d_iord = upload(C->snimg, iord, st);
+    cd* rec = (cd*)C->sst.ensure(per * nang * sizeof(cd));
+    CK(cudaMemcpyAsync(rec, A.t1, per * nang * sizeof(cd), cudaMemcpyHostToDevice, st));
+    const size_t fbytes = (size_t)nang * n * n * sizeof(cd);
+    cd* F = (cd*)Pb.F.ensure(fbytes);
+    CK(cudaMemsetAsync(F, 0, fbytes, st));
+    launch_scatter_records(rec, per, d_first, A.ngr, d_iord, nang, n, F, st);
+  }
   upload(Pb.wnsga2, wnsga2, st);
   Pb.f2.ensure((size_t)nang * n * sizeof(double));
   if (Pb.grid.m) {
