@@ -24,6 +24,7 @@
 
 #include <algorithm>
 #include <stdexcept>
+#include <type_traits>
 
 #include "kernels.h"
 #include "launch_attr.h"
@@ -385,6 +386,8 @@ __global__ void __launch_bounds__(128) k_gj_c1(const BlockArgs g) {
 // accumulator pair is one complex, so a warp reads and writes whole 64-byte pieces of
 // rows), K in chunks of 16 through a 3-stage cp.async ring as the stage product.
 // At K = 64 a tile has 16 K clocks of FP64 tensor work for 131 KB of C read and written.
+// n = 521, 31 angles, first block: 405 us with a row-tile test at every MMA and the complex
+// B values selected in registers (55 % of the FP64 rate), 363 us as it is (61 %).
 constexpr int BM = 64, BN = 64, BK = 16, STAGES = 3;
 constexpr int ASTR = BK + 4, BSTR = BN + 4;
 constexpr int A_TILE = BM * ASTR, B_TILE = BK * BSTR;
@@ -440,6 +443,7 @@ __global__ void __launch_bounds__(128, 2) k_gj_update(const BlockArgs g) {
   }
   // this warp's row tiles with rows below n (none where its columns are past the last)
   const int mlim = bn + wn < total ? min(max(ceil_div(n - bm - wm, 16), 0), 2) : 0;
+  const int flip = (gq & 1) ? 0 : (int)0x80000000;
   cd acc[2][2][8];  // [row tile][row half][4-column group]: lane (g, t) column 4 ni + t
   size_t off[2][2];
 #pragma unroll
@@ -467,29 +471,40 @@ __global__ void __launch_bounds__(128, 2) k_gj_update(const BlockArgs g) {
     else asm volatile("cp.async.commit_group;" ::: "memory");
     const cd* as = As + (kt % STAGES) * A_TILE;
     const cd* bs = Bs + (kt % STAGES) * B_TILE;
-    if (mlim == 0) continue;
+    // whole row tiles only: a test per MMA would keep the next fragments' loads behind it
+    auto chunk = [&](auto tiles) {
+      constexpr int kTiles = decltype(tiles)::value;
 #pragma unroll
-    for (int kk = 0; kk < BK; kk += 4) {
-      cd af[2][2];
+      for (int kk = 0; kk < BK; kk += 4) {
+        cd af[kTiles][2];
 #pragma unroll
-      for (int mi = 0; mi < 2; ++mi)
+        for (int mi = 0; mi < kTiles; ++mi)
 #pragma unroll
-        for (int h = 0; h < 2; ++h)
-          af[mi][h] = as[(wm + mi * 16 + gq + 8 * h) * ASTR + kk + t];
+          for (int h = 0; h < 2; ++h)
+            af[mi][h] = as[(wm + mi * 16 + gq + 8 * h) * ASTR + kk + t];
+        // this lane's column of the (re, im) pairs, and its partner with the sign of i^2
+        const double* brow = reinterpret_cast<const double*>(bs + (kk + t) * BSTR + wn);
 #pragma unroll
-      for (int ni = 0; ni < 8; ++ni) {
-        const cd b = bs[(kk + t) * BSTR + wn + ni * 4 + (gq >> 1)];
-        const double be = (gq & 1) ? b.y : b.x, bo = (gq & 1) ? b.x : -b.y;
+        for (int ni = 0; ni < 8; ++ni) {
+          const double be = brow[8 * ni + gq], bp = brow[8 * ni + (gq ^ 1)];
+          const double bo = __hiloint2double(__double2hiint(bp) ^ flip, __double2loint(bp));
 #pragma unroll
-        for (int mi = 0; mi < 2; ++mi) {
-          if (mi >= mlim) continue;
-          cd& c0 = acc[mi][0][ni];
-          cd& c1 = acc[mi][1][ni];
-          mma64(c0.x, c0.y, c1.x, c1.y, af[mi][0].x, af[mi][1].x, be);
-          mma64(c0.x, c0.y, c1.x, c1.y, af[mi][0].y, af[mi][1].y, bo);
+          for (int mi = 0; mi < kTiles; ++mi) {
+            cd& c0 = acc[mi][0][ni];
+            cd& c1 = acc[mi][1][ni];
+            mma64(c0.x, c0.y, c1.x, c1.y, af[mi][0].x, af[mi][1].x, be);
+          }
+#pragma unroll
+          for (int mi = 0; mi < kTiles; ++mi) {
+            cd& c0 = acc[mi][0][ni];
+            cd& c1 = acc[mi][1][ni];
+            mma64(c0.x, c0.y, c1.x, c1.y, af[mi][0].y, af[mi][1].y, bo);
+          }
         }
       }
-    }
+    };
+    if (mlim == 2) chunk(std::integral_constant<int, 2>{});
+    else if (mlim == 1) chunk(std::integral_constant<int, 1>{});
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
 #pragma unroll
@@ -550,8 +565,8 @@ static bool whole(int n) { return n <= kMaxBlock * kW; }  // one launch
 // clusters fit about one wave, else four.  Whole elimination at n = 521 (one CTA per SM)
 // with 2 / 4 / 6 / 8 sub-panels per block: 1 angle 1.40 / 1.33 / 1.34 / 1.36 ms, 16
 // angles 3.22 / 2.72 / 2.55 / 2.79, 31 angles 4.95 / 4.07 / 4.44 / 4.87, 61 angles 8.28 /
-// 7.73 / 7.93 / 8.47 (one barrier per step since: 1.24, 2.53, 4.01, 7.57; rank-32 updates
-// with physical row swaps and a launch per 16 columns took 4.2, 5.9, 6.8, 10.7 ms).
+// 7.73 / 7.93 / 8.47 (now 1.21, 2.39, 3.74, 7.04; rank-32 updates with physical row swaps
+// and a launch per 16 columns took 4.2, 5.9, 6.8, 10.7 ms).
 static int block_ctas(int nang, int n) {
   const int sub = ceil_div(n, kW);
   if (whole(n)) return sub;
