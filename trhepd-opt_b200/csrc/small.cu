@@ -38,22 +38,27 @@ namespace fused {
 constexpr int kThreads = 128;
 constexpr int kTabBufs = 4;  // table columns in flight where shared memory allows
 
-// RT row tiles; GW column groups per warp.
-template <int RT, int GW>
+// RT row tiles; GW column groups per warp.  kRk4: the classical RK4 steps of rk4_int
+// (surf_rk.f90:27-91) instead of the RKN kicks: Q, P, the stage point's Q and the two
+// weighted sums in shared memory (elements of them touched by their own lane only), the
+// stage point's P in registers.
+template <int RT, int GW, bool kRk4>
 struct Cfg {
   static constexpr int NP = 16 * RT;
   static constexpr int WC = RT == 2 ? 2 : 4;        // warps along the columns
   static constexpr int WR = 4 / WC;                 // and along the row tiles
   static constexpr int TW = RT / WR;                // row tiles per warp
   static constexpr int KS = 4 * RT;                 // k steps of a product
-  static constexpr bool PREG = RT <= 3;             // P in registers
-  static constexpr int QB = RT <= 2 ? 2 : 1;        // Q buffers (one barrier per stage less)
+  static constexpr bool PREG = RT <= 3 && !kRk4;    // P in registers
+  static constexpr int QB = RT <= 2 && !kRk4 ? 2 : 1;  // Q buffers (one barrier per stage less)
   static constexpr int STR = NP + 4;                // 4 mod 8 complex: conflict-free fragments
-  static constexpr int MINB = RT <= 2 ? 3 : RT == 3 ? 2 : 1;
-  // complex values of Q, P and the pivot rows, and the fragment codes (8 bytes per lane
-  // and k step)
+  static constexpr int MINB = kRk4 ? (RT <= 2 ? 2 : 1) : RT <= 2 ? 3 : RT == 3 ? 2 : 1;
+  // complex values of Q, P, the RK4 arrays or else the pivot rows (which share the first
+  // RK4 sum: it is dead at the end of a slice), and the fragment codes (8 bytes per lane and
+  // k step)
+  static constexpr size_t extra = kRk4 ? (size_t)3 * NP * STR : (size_t)16 * STR;
   static constexpr size_t elems =
-      (size_t)(QB + (PREG ? 0 : 1)) * NP * STR + 16 * STR + KS * kThreads / 2;
+      (size_t)(QB + (PREG ? 0 : 1)) * NP * STR + extra + KS * kThreads / 2;
 };
 
 __device__ __forceinline__ unsigned smem_addr(const void* p) {
@@ -89,10 +94,10 @@ __device__ __forceinline__ void fmma(cd& c0, cd& c1, double a0, double a1, doubl
       : "d"(a0), "d"(a1), "d"(b0));
 }
 
-template <int RT, int GW>
-__global__ void __launch_bounds__(kThreads, Cfg<RT, GW>::MINB)
+template <int RT, int GW, bool kRk4>
+__global__ void __launch_bounds__(kThreads, Cfg<RT, GW, kRk4>::MINB)
     k_fused_rkn(const __grid_constant__ FusedLaunch L, int nbuf, int tab_stride) {
-  using C = Cfg<RT, GW>;
+  using C = Cfg<RT, GW, kRk4>;
   constexpr int NP = C::NP, STR = C::STR, TW = C::TW;
   // this CTA's problem: the last whose first CTA is <= blockIdx.x
   int pi = 0;
@@ -104,8 +109,11 @@ __global__ void __launch_bounds__(kThreads, Cfg<RT, GW>::MINB)
   cd* Qo = Qs + (C::QB - 1) * NP * STR;                 // the other (the same for QB = 1)
   cd* const Ps = Qs + C::QB * NP * STR;                 // PREG = false only
   cd* const c1s = Ps + (C::PREG ? 0 : NP * STR);        // 16 pivot rows
-  uint2* const codes = reinterpret_cast<uint2*>(c1s + 16 * STR);  // [KS][kThreads]
-  cd* const tab = c1s + 16 * STR + C::KS * kThreads / 2;          // [nbuf][tab_stride]
+  cd* const SQ = c1s;                                   // kRk4 only, as the next two
+  cd* const SP = SQ + NP * STR;
+  cd* const Qt = SP + NP * STR;
+  uint2* const codes = reinterpret_cast<uint2*>(c1s + C::extra);  // [KS][kThreads]
+  cd* const tab = c1s + C::extra + C::KS * kThreads / 2;          // [nbuf][tab_stride]
   __shared__ double csum[kThreads];
   __shared__ double red_d[2][4];
   __shared__ unsigned keys[2][32];
@@ -133,6 +141,7 @@ __global__ void __launch_bounds__(kThreads, Cfg<RT, GW>::MINB)
     const bool ok = i < n && j < n;
     Qs[e] = ok ? Qg[(size_t)i * ld + j] : cd{0.0, 0.0};
     if (C::QB == 2) Qo[e] = cd{0.0, 0.0};
+    if (kRk4) Qt[e] = cd{0.0, 0.0};
   }
   double dreg[GW];
 #pragma unroll
@@ -208,13 +217,9 @@ __global__ void __launch_bounds__(kThreads, Cfg<RT, GW>::MINB)
     }
   };
   for (int c = 0; c < max(nbuf - 1, 1); ++c) fetch();
-  // P += cb (Q V + Q o D), Q <- Q + ca P with the next table column; ends without a barrier
-  auto stage = [&](double cb, double ca) {
-    const cd* tc = tab + out * tab_stride;
-    arrived();
-    __syncthreads();  // Q is there too
-    if (nbuf > 1) fetch();
-    cd acc[TW][2][GW];
+  cd acc[TW][2][GW];
+  // acc = -Qin V with the column at tc
+  auto product = [&](const cd* Qin, const cd* tc) {
 #pragma unroll
     for (int i = 0; i < TW; ++i)
 #pragma unroll
@@ -229,7 +234,7 @@ __global__ void __launch_bounds__(kThreads, Cfg<RT, GW>::MINB)
 #pragma unroll
       for (int i = 0; i < TW; ++i)
 #pragma unroll
-        for (int h = 0; h < 2; ++h) x[i][h] = Qs[(row0 + 16 * i + 8 * h) * STR + 4 * ks + t4];
+        for (int h = 0; h < 2; ++h) x[i][h] = Qin[(row0 + 16 * i + 8 * h) * STR + 4 * ks + t4];
 #pragma unroll
       for (int j = 0; j < GW; ++j) {
         const unsigned w = j < 2 ? code.x : code.y, cj = (j & 1) ? w >> 16 : w & 0xffffu;
@@ -259,6 +264,14 @@ __global__ void __launch_bounds__(kThreads, Cfg<RT, GW>::MINB)
       load(min(ks + 2, C::KS - 1), af[0], bf[0]);
       mma(af[1], bf[1]);
     }
+  };
+  // P += cb (Q V + Q o D), Q <- Q + ca P with the next table column; ends without a barrier
+  auto stage = [&](double cb, double ca) {
+    const cd* tc = tab + out * tab_stride;
+    arrived();
+    __syncthreads();  // Q is there too
+    if (nbuf > 1) fetch();
+    product(Qs, tc);
     if (C::QB == 1 || nbuf == 1) __syncthreads();  // every read of Q and the column done
     if (nbuf == 1) fetch();
 #pragma unroll
@@ -497,22 +510,74 @@ __global__ void __launch_bounds__(kThreads, Cfg<RT, GW>::MINB)
       }
   };
 
-  for (int l = 1; l <= ns; ++l) {
-    for (int k = 1; k <= s; ++k) {
-      // k == 1 merges the end-of-slice half kick of slice l-1 with the first kick
-      const double cb = (k == 1) ? (l == 1 ? 1.0 : 2.0) * L.bab[0] * dz : L.bab[2 * k - 2] * dz;
-      stage(cb, L.bab[2 * k - 1] * dz);
-    }
-    const bool last = l == ns;
-    bool renorm = last;
-    if (!last) renorm = (L.policy == 0) ? needs_renorm() : (l % a.interval) == 0;
+  auto end_of_slice = [&](int l) {
+    bool renorm = l == ns;
+    if (!renorm) renorm = (L.policy == 0) ? needs_renorm() : (l % a.interval) == 0;
     if (renorm) {
       __syncthreads();
       gauss_jordan();
     }
+  };
+  if constexpr (kRk4) {
+    // stage j: weight of k_j in the sum, step to the next stage point; the middle column
+    // serves two stages, the last one the next slice's first
+    cd pt[TW * 2 * GW];
+    const cd* tc = nullptr;
+    for (int l = 1; l <= ns; ++l) {
+#pragma unroll 1
+      for (int st = 0; st < 4; ++st) {
+        const double w = (st == 1 || st == 2) ? 2.0 : 1.0, step = st < 2 ? 0.5 * dz : dz;
+        const bool next = (st & 1) || (st == 0 && l == 1);
+        if (next) {
+          tc = tab + out * tab_stride;
+          arrived();
+        }
+        __syncthreads();  // the stage point is there
+        if (next) fetch();
+        const cd* Qin = st == 0 ? Qs : Qt;
+        product(Qin, tc);
+        __syncthreads();  // every read of the stage point done
+#pragma unroll
+        for (int i = 0; i < TW; ++i)
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int j = 0; j < GW; ++j) {
+              const int o = (row0 + 16 * i + 8 * h) * STR + col(j);
+              cd& ps = pt[(i * 2 + h) * GW + j];
+              const cd q = Qin[o], z = acc[i][h][j], p0 = Ps[o];  // z = -Q V
+              const cd kp = cd{fma(q.x, dreg[j], -z.x), fma(q.y, dreg[j], -z.y)};
+              const cd kq = st == 0 ? p0 : ps;
+              cd sq = kq, sp = kp;
+              if (st > 0) {
+                sq = SQ[o] + w * kq;
+                sp = SP[o] + w * kp;
+              }
+              if (st < 3) {
+                SQ[o] = sq;
+                SP[o] = sp;
+                Qt[o] = Qs[o] + step * kq;
+                ps = p0 + step * kp;
+              } else {
+                Qs[o] = Qs[o] + (dz / 6) * sq;
+                Ps[o] = p0 + (dz / 6) * sp;
+              }
+            }
+      }
+      end_of_slice(l);
+    }
+  } else {
+    for (int l = 1; l <= ns; ++l) {
+      for (int k = 1; k <= s; ++k) {
+        // k == 1 merges the end-of-slice half kick of slice l-1 with the first kick
+        const double cb = (k == 1) ? (l == 1 ? 1.0 : 2.0) * L.bab[0] * dz : L.bab[2 * k - 2] * dz;
+        stage(cb, L.bab[2 * k - 1] * dz);
+      }
+      end_of_slice(l);
+    }
+    // final half kick with Q = I: P += b1 dz M(end)
+    stage(L.bab[0] * dz, 0.0);
   }
-  // final half kick with Q = I: P += b1 dz M(end)
-  stage(L.bab[0] * dz, 0.0);
   if (tid == 0 && dead)  // copies still on their way (as long as they may take)
     while (consumed < issued) {
       wait_parity(&bars[out], parity);
@@ -538,27 +603,40 @@ __global__ void __launch_bounds__(kThreads, Cfg<RT, GW>::MINB)
       }
 }
 
-template <int RT, int GW>
-void launch(const FusedLaunch& L, int nvmax, cudaStream_t st) {
-  using C = Cfg<RT, GW>;
-  static SmemOptIn attr;
-  const int stride = 2 * (nvmax + 1);
-  // four column buffers where they leave the CTAs per SM the registers allow, else one or
-  // two (a column's copy takes longer than a stage of a small problem)
+// Shared memory of a launch: four column buffers where they leave the CTAs per SM the
+// registers allow, else two or one (a column's copy takes longer than a stage of a small
+// problem).
+template <int RT, int GW, bool kRk4>
+int buffers(int stride, size_t& smem) {
+  using C = Cfg<RT, GW, kRk4>;
   auto bytes = [&](int b) { return (C::elems + (size_t)b * stride) * sizeof(cd); };
   int nbuf = bytes(kTabBufs) <= size_t(227 * 1024) / C::MINB - 4096 ? kTabBufs : 2;
   if (bytes(nbuf) > 224 * 1024) nbuf = 1;
-  const size_t smem = (C::elems + (size_t)nbuf * stride) * sizeof(cd);
-  attr.ensure((const void*)k_fused_rkn<RT, GW>, smem);
-  k_fused_rkn<RT, GW><<<L.total_ctas, kThreads, smem, st>>>(L, nbuf, stride);
+  smem = bytes(nbuf);
+  return smem <= 224 * 1024 ? nbuf : 0;
+}
+
+template <int RT, int GW, bool kRk4 = false>
+bool launch(const FusedLaunch& L, int nvmax, cudaStream_t st) {
+  static SmemOptIn attr;
+  const int stride = 2 * (nvmax + 1);
+  size_t smem = 0;
+  const int nbuf = buffers<RT, GW, kRk4>(stride, smem);
+  if (nbuf < (kRk4 ? 2 : 1)) return false;  // RK4 keeps a column through two stages
+  attr.ensure((const void*)k_fused_rkn<RT, GW, kRk4>, smem);
+  k_fused_rkn<RT, GW, kRk4><<<L.total_ctas, kThreads, smem, st>>>(L, nbuf, stride);
+  return true;
 }
 
 }  // namespace fused
 
-int launch_fused_rkn(const FusedLaunch& L, cudaStream_t st) {
+namespace {
+// Checks a launch; returns the largest beam and entry counts.
+void check(const FusedLaunch& L, int& nmax, int& nvmax) {
   if (L.nprob < 1 || L.nprob > kFusedMaxProblems || L.s < 1 || L.s > 11)
     throw std::invalid_argument("fused integration: bad launch");
-  int nmax = 0, nvmax = 0, ctas = 0;
+  int ctas = 0;
+  nmax = nvmax = 0;
   for (int q = 0; q < L.nprob; ++q) {
     const FusedProblem& a = L.p[q];
     if (a.n < 2 || a.n > kFusedMaxBeams || a.ns < 1 || a.interval < 1 || a.nang < 1 ||
@@ -569,16 +647,40 @@ int launch_fused_rkn(const FusedLaunch& L, cudaStream_t st) {
     nvmax = std::max(nvmax, a.nv);
   }
   if (ctas != L.total_ctas) throw std::invalid_argument("fused integration: CTA count");
-  if (nmax <= 16)
-    fused::launch<1, 1>(L, nvmax, st);
-  else if (nmax <= 24)
-    fused::launch<2, 3>(L, nvmax, st);
-  else if (nmax <= 32)
-    fused::launch<2, 4>(L, nvmax, st);
-  else if (nmax <= 48)
-    fused::launch<3, 3>(L, nvmax, st);
-  else
-    fused::launch<4, 4>(L, nvmax, st);
+}
+}  // namespace
+
+int launch_fused_rkn(const FusedLaunch& L, cudaStream_t st) {
+  int nmax = 0, nvmax = 0;
+  check(L, nmax, nvmax);
+  const bool ok = nmax <= 16   ? fused::launch<1, 1>(L, nvmax, st)
+                  : nmax <= 24 ? fused::launch<2, 3>(L, nvmax, st)
+                  : nmax <= 32 ? fused::launch<2, 4>(L, nvmax, st)
+                  : nmax <= 48 ? fused::launch<3, 3>(L, nvmax, st)
+                               : fused::launch<4, 4>(L, nvmax, st);
+  if (!ok) throw std::invalid_argument("fused integration: shared memory");
+  return 1;
+}
+
+bool fused_rk4_fits(int n, int nv) {
+  size_t smem = 0;
+  const int stride = 2 * (nv + 1);
+  return n >= 2 && n <= kFusedRk4MaxBeams && nv >= 1 && nv <= kFusedMaxEntries &&
+         (n <= 16   ? fused::buffers<1, 1, true>(stride, smem)
+          : n <= 24 ? fused::buffers<2, 3, true>(stride, smem)
+          : n <= 32 ? fused::buffers<2, 4, true>(stride, smem)
+                    : fused::buffers<3, 3, true>(stride, smem)) >= 2;
+}
+
+int launch_fused_rk4(const FusedLaunch& L, cudaStream_t st) {
+  int nmax = 0, nvmax = 0;
+  check(L, nmax, nvmax);
+  if (L.s != 2 || !fused_rk4_fits(nmax, nvmax))
+    throw std::invalid_argument("fused RK4: unsupported problem");
+  if (nmax <= 16) fused::launch<1, 1, true>(L, nvmax, st);
+  else if (nmax <= 24) fused::launch<2, 3, true>(L, nvmax, st);
+  else if (nmax <= 32) fused::launch<2, 4, true>(L, nvmax, st);
+  else fused::launch<3, 3, true>(L, nvmax, st);
   return 1;
 }
 

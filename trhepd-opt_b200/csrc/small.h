@@ -45,4 +45,10 @@ struct FusedLaunch {
 // the number of kernels launched.
 int launch_fused_rkn(const FusedLaunch& L, cudaStream_t st);
 
+// The same for classical RK4 (rk4_int, surf_rk.f90:27-91; L.s = 2 table columns per slice,
+// L.bab unused).  Its five arrays fit one SM up to 48 beams and, there, 278 table entries.
+constexpr int kFusedRk4MaxBeams = 48;
+bool fused_rk4_fits(int n, int nv);
+int launch_fused_rk4(const FusedLaunch& L, cudaStream_t st);
+
 }  // namespace trhepd

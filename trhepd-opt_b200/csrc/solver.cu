@@ -757,6 +757,24 @@ FusedProblem fused_problem(const RunState& R, double dz, int first_cta) {
   return f;
 }
 
+// A whole integration in one launch, state in shared memory (small.cu).
+void fused_launch(trhepd_context* C, trhepd_problem& Pb, RunState& R,
+                  int (*launch)(const FusedLaunch&, cudaStream_t)) {
+  const Integrator& I = Pb.I;
+  static thread_local FusedLaunch L;  // 17 KB of kernel parameters
+  L.nprob = 1;
+  L.s = I.s;
+  L.policy = C->renorm_policy;
+  L.total_ctas = R.nang;
+  for (int q = 0; I.bab && q < 2 * I.s + 1; ++q) L.bab[q] = I.bab[q];
+  L.p[0] = fused_problem(R, Pb.dz, 0);
+  const cudaEvent_t* ev = C->profile ? &C->evpool[0] : nullptr;  // the launch is one entry
+  for (int e = 0; ev && e < 2; ++e) CK(cudaEventRecord(ev[e], R.st));
+  R.launches += launch(L, R.st);
+  for (int e = 2; ev && e < 4; ++e) CK(cudaEventRecord(ev[e], R.st));
+  if (ev) R.prof_entries = 1;
+}
+
 // Symplectic RKN (hp_int_spa, surf_prkn.f90:278-330) batched over angles.
 void run_rkn(trhepd_context* C, trhepd_problem& Pb, int precision, RunState& R) {
   const Integrator& I = Pb.I;
@@ -765,25 +783,7 @@ void run_rkn(trhepd_context* C, trhepd_problem& Pb, int precision, RunState& R) 
   const bool every_slice = (Pb.n == 1 && Pb.int_method == 6);  // hp_int_spa1d renormalises each slice
   if (!R.split && R.nprob == 1 && Pb.n >= 2 && Pb.n <= std::min(C->fused_max_n, kFusedMaxBeams) &&
       Pb.nv <= kFusedMaxEntries) {
-    // whole integration in one launch, state in shared memory (small.cu)
-    static thread_local FusedLaunch L;  // 17 KB of kernel parameters
-    L.nprob = 1;
-    L.s = I.s;
-    L.policy = C->renorm_policy;
-    L.total_ctas = R.nang;
-    for (int q = 0; q < 2 * I.s + 1; ++q) L.bab[q] = I.bab[q];
-    L.p[0] = fused_problem(R, dz, 0);
-    const cudaEvent_t* ev = C->profile ? &C->evpool[0] : nullptr;  // the launch is one entry
-    if (ev) {
-      CK(cudaEventRecord(ev[0], R.st));
-      CK(cudaEventRecord(ev[1], R.st));
-    }
-    R.launches += launch_fused_rkn(L, R.st);
-    if (ev) {
-      CK(cudaEventRecord(ev[2], R.st));
-      CK(cudaEventRecord(ev[3], R.st));
-      R.prof_entries = 1;
-    }
+    fused_launch(C, Pb, R, launch_fused_rkn);
     R.products += (long)I.s * R.ns - 1;
     R.renorms += (C->renorm_policy == 1) ? (R.ns - 1) / R.interval : R.ns - 1;
     finish_device(C, Pb, R);
@@ -869,6 +869,13 @@ void run_lf(trhepd_context* C, trhepd_problem& Pb, int precision, RunState& R) {
 void run_rk4(trhepd_context* C, trhepd_problem& Pb, int precision, RunState& R) {
   const double dz = Pb.dz;
   begin_run(C, Pb, precision, 4 * Pb.ns, R, context_workspace(C));
+  if (!R.split && !Pb.I.gs && Pb.n <= C->fused_max_n && fused_rk4_fits(Pb.n, Pb.nv)) {
+    fused_launch(C, Pb, R, launch_fused_rk4);
+    R.products += 4L * R.ns;
+    R.renorms += (C->renorm_policy == 1) ? (R.ns - 1) / R.interval : R.ns - 1;
+    finish_device(C, Pb, R);
+    return;
+  }
   const size_t sb = R.sbytes;
   cd* Qt = (cd*)C->rk[0].ensure(sb);
   cd* Pt = (cd*)C->rk[1].ensure(sb);
