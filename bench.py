@@ -5,17 +5,17 @@ Workload (default ``dense521``): synthetic 2x2 Si/Ge surface over a 4-atom
 bulk, N = 521 beams, 61 glancing angles (0.5..6.5 deg), 2004 slices of
 0.01 A, symplectic RKN-4 (int_method 5).  One step = one solve of all 61 angles.
 
-* ``value``: the split-precision form (default: 5 signed 8-bit digit slices per
-  operand, 39 bits, on tcgen05 kind::i8 with exact INT32 accumulation; every
-  spot within 1e-6 relative of FP64 at N = 521; ``--precision``
-  bf16 / fp64 select the other forms), inputs resident in HBM
+* ``value``: the split-precision form (``--precision`` bf16 / fp64 select the other
+  forms; beams on a dense index grid, as this workload's, take the FP64 convolution
+  stage products in every form, other beam sets 5 signed 8-bit digit slices per
+  operand on tcgen05 kind::i8), inputs resident in HBM
   (trhepd_problem_solve), device time from CUDA events on the library stream,
   max over ranks.
 * ``e2e``: the same metric through the C ABI with host buffers
   (trhepd_srfref: uploads, stage-table build, solve, intensities back).
 * ``fp64``: the plain FP64 form of the same workload, its speed and the split
   form's error against it; ``bf16_split``: the BF16-slice form beside it.
-* ``roofline``: the tensor-core stage kernel, live event timing of every launch.
+* ``roofline``: the stage kernel, live event timing of every launch.
 * ``cpu_baseline``: the CPU oracle (C++ restatement of the reference path,
   OpenMP over angles, OpenBLAS) on a bounded sample of the workload.
 
@@ -507,12 +507,14 @@ def main():
     ms_per_step = max_ms / args.steps
     _, f2_main = rp.fetch()
 
-    # ---- roofline of the tensor-core stage kernel (one profiled solve): CUDA events
-    # around every launch of that kernel on the library stream
+    # ---- roofline of the stage kernel (one profiled solve): CUDA events around every
+    # launch of that kernel on the library stream
     ctx.set_option(native.OPT_PROFILE, 1)
     stp = solve_ms(prec)
     ctx.set_option(native.OPT_PROFILE, 0)
     nprod = max(stp["stage_products"], 1)
+    # a dense product takes a launch or more, the convolutions one for many stages
+    convolved = stp["launches"] < stp["stage_products"]
     tensor_ms = stp["tensor_kernel_ms"] / nprod
     stage_ms = stp["stage_kernel_ms"] / nprod
     fp64_equiv = 8.0 * nang * n ** 3  # complex N x N x N product per angle
@@ -561,7 +563,7 @@ def main():
         mma_issue = 2 * 8192 * sms * clk["sm_mhz"] * 1e6 / 1e12   # TOP/s
     traffic = NCU_TRAFFIC.get((args.workload, form, slices))
     tensor_floor_ms = issued / (peak * 1e12) * 1e3 if peak else 0.0
-    roof = {"bound": "tensor" if tensor_floor_ms >= hbm_ms else "hbm",
+    roof = convolution_roofline(stp, sp, nang, n, f64_peak) if convolved else {"bound": "tensor" if tensor_floor_ms >= hbm_ms else "hbm",
             "achieved": achieved, "peak": peak, "unit": unit,
             "frac": (achieved / peak) if peak else None,
             "traffic": (traffic * nang / 16.0) if traffic else None,
@@ -623,8 +625,10 @@ def main():
         _, f2_64 = rp.fetch()
         fp64 = {"value": nang / (st["device_ms"] / 1e3), "ms_per_step": st["device_ms"],
                 "split_speedup": (st["device_ms"] / ms_per_step),
-                "roofline": fp64_roofline(st64p, nang, n, f64_peak, peaks,
-                                          NCU_TRAFFIC.get((args.workload, "fp64", 0))),
+                "roofline": convolution_roofline(st64p, sp, nang, n, f64_peak)
+                if st64p["launches"] < st64p["stage_products"] else
+                fp64_roofline(st64p, nang, n, f64_peak, peaks,
+                              NCU_TRAFFIC.get((args.workload, "fp64", 0))),
                 "breakdown": {"solve_ms": st64p["device_ms"],
                               "stage_products_ms": st64p["stage_kernel_ms"],
                               "renormalisations_ms": st64p["renorm_ms"],
@@ -687,14 +691,17 @@ def main():
         line = {"metric": METRIC, "value": value, "unit": "angle-solves/s", "n_gpus": ws,
                 "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms_per_step,
                 "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-                "dtype": {native.SPLIT_INT8: f"i8x{slices}-split/f64",
-                          native.SPLIT_BF16: f"bf16x{slices}-split/f64", native.FP64: "f64"}[prec],
+                "dtype": "f64" if convolved else {native.SPLIT_INT8: f"i8x{slices}-split/f64",
+                                                  native.SPLIT_BF16: f"bf16x{slices}-split/f64",
+                                                  native.FP64: "f64"}[prec],
                 "data": "synthetic",
                 "config": {"workload": desc, "nb": n, "nangles": nang, "slices": rp.ns,
                            "precision": {native.SPLIT_INT8: "split-int8",
                                          native.SPLIT_BF16: "split-bf16",
                                          native.FP64: "fp64"}[prec],
                            "split_slices": slices if split else None,
+                           "stage_products": "FP64 convolutions over the beam grid" if convolved
+                           else "dense products",
                            "renormalisation": "growth bound ln(1e3)",
                            "renormalisations_per_solve": stp["renormalisations"],
                            "stage_products_per_solve": stp["stage_products"],
@@ -720,15 +727,44 @@ def main():
                     "max_rel_err_all_spots": fp64["split_max_rel_err_all_spots"],
                     "every_spot_within_1e-6": bool(fp64["split_max_rel_err_all_spots"] <= 1e-6),
                     "fp64_value": fp64["value"], "split_value": value,
-                    "renormalisation": "growth bound ln(1e3) for both forms; Gauss-Jordan "
-                                       "panels of 16 columns (row-per-thread panel kernel) "
-                                       "with the trailing update on the FP64 tensor path in "
-                                       "both forms; panel arithmetic with fused complex "
-                                       "multiply-adds (split) or products formed first (FP64)"}}
+                    "renormalisation": "growth bound ln(1e3) and the same cluster elimination "
+                                       "on the FP64 tensor path for both forms"}}
         print(json.dumps(line), flush=True)
     if pg:
         pg.barrier()
         pg.destroy_process_group()
+
+
+def convolution_roofline(stp: dict, sp, nang: int, n: int, f64_peak) -> dict:
+    """Roofline of k_conv_stages from one profiled solve: the floating-point operations of
+    its transforms per stage (5 m log2 m per m-point transform, m >= the beams' index
+    spans: 2 per line and 8 per column there and back, 6 per spectrum point, 6 per parity
+    turn, 10 per beam's update) against cuBLAS DGEMM measured in the run.  DFT arithmetic
+    is half additions, so the FP64 pipe is fuller than the fraction says; the state stays
+    on chip between renormalisations, so HBM does not bound it."""
+    import ctypes
+    import math
+
+    def ints(ptr):
+        return np.frombuffer(ctypes.string_at(ptr, 4 * n), np.int32)
+    spans = []
+    for shear in range(-2, 3):
+        for a, b in ((ints(sp.args.ih), ints(sp.args.ik)), (ints(sp.args.ik), ints(sp.args.ih))):
+            v = b + shear * a
+            spans.append((max(int(np.ptp(a)), int(np.ptp(v))) + 1, int(np.ptp(a)) + 1))
+    span = min(spans)[0]
+    m = next(k for k in (9, 10, 12, 15, 16, 20, 25, 27, 32) if k >= span)
+    fft = 5.0 * m * math.log2(m)
+    row = (4 * span + 8 * m) * fft + 6.0 * 4 * m * m + 6.0 * m * (2 * span + 4 * m) + 10.0 * n
+    ms = stp["tensor_kernel_ms"] / max(stp["stage_products"], 1)
+    achieved = nang * n * row / (ms * 1e-3) / 1e12
+    peak = f64_peak["sustained"] if f64_peak else None
+    return {"bound": "fp64", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
+            "frac": achieved / peak if peak else None,
+            "kernel": f"k_conv_stages<{m}> (FP64 DFT convolutions, state in shared memory)",
+            "peak_source": "cuBLAS DGEMM 8192^3 measured in this run, sustained over a 3 s loop",
+            "avg_stage_ms": ms, "flop_per_stage": nang * n * row, "transform_length": m,
+            "dense_equivalent_tflops": 8.0 * nang * n ** 3 / (ms * 1e-3) / 1e12}
 
 
 def fp64_roofline(stp: dict, nang: int, n: int, f64_peak, peaks: dict, traffic) -> dict:
@@ -769,7 +805,8 @@ def surface_slices(workdir: Path, s) -> int:
 
 def h2d_bytes(sp, rp) -> int:
     """Bytes trhepd_srfref copies host->device per call: the mod_scpot3 arrays, the
-    stage depths, the beam-pair map and the per-angle gammas, energies and bulk f."""
+    stage depths, the beam-pair map, the per-angle gammas and energies and the bulk
+    records (the beam grid's few tables are left out)."""
     p = sp.pot
     natm = p.natms + p.natmb
     b = 8 * (p.nv * 6 * p.nelm + 6 * p.nelm + p.nelm + p.nv)        # asf, b, dchg, Ghk
@@ -777,7 +814,9 @@ def h2d_bytes(sp, rp) -> int:
     b += 16 * (p.nv * p.natms + 2 * p.nvb * p.natmb)                 # st0, st1, st2
     b += 8 * rp.ncol + 4 * rp.nb * rp.nb                             # depths, pair map
     ld = -(-rp.nb // 16) * 16
-    b += rp.nangles * (16 * rp.nb + 16 * ld + 16 * rp.nb * rp.nb + 8)  # gam, D, F, w
+    import ctypes
+    nbg = np.frombuffer(ctypes.string_at(sp.args.nbg, 4 * sp.args.ngr), np.int32).astype(int)
+    b += rp.nangles * (16 * rp.nb + 16 * ld + 16 * int((nbg ** 2).sum()) + 8)  # gam, D, f, w
     del natm
     return int(b)
 

@@ -32,7 +32,9 @@ enum trhepd_status {
   TRHEPD_EIO = 6          /* input file missing or malformed */
 };
 
-/* precision forms of the surface solve */
+/* precision forms of the surface solve.  Where the beams lie on a dense index grid (nb >
+   64) the stage products are FP64 convolutions in every form (with 3 or 4 slices only up
+   to spans of 20); the digit slices are the split forms' products elsewhere. */
 enum trhepd_precision {
   TRHEPD_FP64 = 0,        /* all-FP64 (DMMA) */
   TRHEPD_SPLIT_BF16 = 1,  /* stage products from BF16 slices on tcgen05 (FP32 accumulators),
