@@ -33,8 +33,8 @@ enum trhepd_status {
 };
 
 /* precision forms of the surface solve.  Where the beams lie on a dense index grid (nb >
-   64) the stage products are FP64 convolutions in every form (with 3 or 4 slices only up
-   to spans of 20); the digit slices are the split forms' products elsewhere. */
+   64) the stage products are FP64 convolutions in the FP64 form, and in the split forms
+   too where those are faster than their digit slices. */
 enum trhepd_precision {
   TRHEPD_FP64 = 0,        /* all-FP64 (DMMA) */
   TRHEPD_SPLIT_BF16 = 1,  /* stage products from BF16 slices on tcgen05 (FP32 accumulators),

@@ -75,7 +75,7 @@ def solve(tool, beams, pair):
 
 
 SETS = {"disc66": disc(66), "disc95-shuffled": disc(95, seed=1), "disc131-sheared": disc(131, 2, 2),
-        "disc191-sheared-back": disc(191, 3, -1), "wide80": disc(80, 4, scale=(1, 3)),
+        "disc191-sheared-back": disc(191, 3, -1), "wide100": disc(100, 4, scale=(1, 2)),
         "holes300": [b for i, b in enumerate(disc(340, 5)) if i % 9], "disc521": disc(521, 6),
         "disc640": disc(640)}
 

@@ -455,14 +455,17 @@ Workspace context_workspace(trhepd_context* C) {
 }
 
 // Whether the stage products of a solve are convolutions over the beam grid.  Against the
-// dense FP64 products they always pay where conv_grid returns a grid (n = 521, 16 angles:
-// 0.68 -> 0.17 ms per stage; n = 95, 61 angles: 56 -> 14.5 us).  Against the digit products
-// with 5 slices too (n = 521, 31 angles: 0.37 -> 0.31 ms; n = 191, 61 angles: 103 -> 54
-// us); 3 and 4 slices have 6 and 10 slice pairs instead of 15 and stay ahead on the
-// largest grids.
+// dense FP64 products they pay wherever conv_grid returns a grid (n = 521, 16 angles: 0.68
+// -> 0.17 ms per stage; n = 95, 61 angles: 56 -> 14.5 us).  Against the digit products (5
+// slices) they do on short transforms (n = 191, 61 angles, m = 15: 103 -> 62 us, 87 with 3
+// slices) and on well filled longer ones (31 angles, n = 521, m = 27: 376 -> 343 us; 61
+// angles, n = 300, m = 20: 225 -> 189), not below (n = 400, m = 25: 219 against 251; n = 250,
+// m = 25: 102 against 157) nor with fewer slices (n = 521, 4 slices: 330).
 bool use_convolution(const trhepd_context* C, const trhepd_problem& Pb, bool split) {
-  if (!Pb.grid.m || Pb.I.family > kRk4) return false;
-  return !split || C->split_slices >= 5 || Pb.grid.m <= 20;
+  const int m = Pb.grid.m;
+  if (!m || Pb.I.family > kRk4) return false;
+  if (!split || m <= 16) return true;
+  return C->split_slices >= 5 && m <= 27 && (double)Pb.n >= 0.7 * m * m;
 }
 
 void begin_run(trhepd_context* C, trhepd_problem& Pb, int precision, int nprod_max, RunState& R,
