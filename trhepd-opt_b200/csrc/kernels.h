@@ -93,8 +93,17 @@ constexpr int kMaxBeams = 832;
 //   kGjFp64, kGjFused  the surface solve: clusters and the FP64 tensor path
 //                    (renorm.cu) up to kGjClusterMaxRows beams; beyond, the
 //                    shared-memory panels with products first (the FP64 form) or
-//                    four fused multiply-adds per complex product (the split forms).
-enum GjArith { kGjProductFirst = 0, kGjFused = 1, kGjFp64 = 2 };
+//                    four fused multiply-adds per complex product (the split forms),
+//   kGjFp64Rows, kGjFusedRows  the renormalisations of solves that amplify a change of
+//                    rounding: row swaps and a row per thread up to kGjClusterMaxRows
+//                    beams, the shared-memory panels beyond.
+enum GjArith {
+  kGjProductFirst = 0,
+  kGjFused = 1,
+  kGjFp64 = 2,
+  kGjFusedRows = 3,
+  kGjFp64Rows = 4
+};
 constexpr int kGjClusterMaxRows = 640;
 size_t gj_scratch_bytes(int nang, int n);
 int launch_gauss_jordan(cd* Q, cd* P, const int* flag, int nang, int n, int ld, void* scratch,

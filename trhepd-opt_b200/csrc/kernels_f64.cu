@@ -414,29 +414,36 @@ void launch_set_identity(cd* Q, const int* flag, int nang, int n, int ld, cudaSt
 // ============================================================ K8 blocked Gauss-Jordan
 // [Q | P] -> [I | Q^{-1} P] with partial pivoting (pivot = max |re|+|im| among the
 // rows not yet used, lowest index on ties, as zgetrf's izamax), in panels of
-// kW = 16 columns: the shared-memory path, for the bulk solve (products formed first)
-// and for more than kGjClusterMaxRows rows; the other solves take renorm.cu.  The
-// panel kernel factors rows c0.. of the n x 16 panel in shared memory (LU with row
-// swaps) and forms W1 = B1^{-1} and the elimination multipliers L2 = B2 B1^{-1}
-// for every other row; the update kernel applies the swaps and
-//   C1 <- W1 C1,   C2 <- C2 - L2 C1
-// to all remaining columns (Q columns right of the panel and every P column),
-// one thread per column.
+// kW = 16 columns.  Two implementations beside renorm.cu's:
+// * shared memory (the bulk solve, the boundary transforms of the solves below, and
+//   more than kGjClusterMaxRows rows): the panel kernel factors rows c0.. of the
+//   n x 16 panel in shared memory (LU with row swaps) and forms W1 = B1^{-1} and the
+//   elimination multipliers L2 = B2 B1^{-1} for every other row; the update kernel
+//   applies the swaps and C1 <- W1 C1, C2 <- C2 - L2 C1 to all remaining columns (Q
+//   columns right of the panel and every P column), one thread per column.
+// * row per thread (the renormalisations of solves that amplify a change of rounding,
+//   solver.cu: rounding_amplified): k_gj_panel_rows eliminates the panel in place with
+//   each row in one thread's registers and writes E; the trailing update C' = C + E C1
+//   runs on the FP64 tensor path (k_gj_update_mma), rank 32 in the split forms.  It
+//   takes 1.8 to 3.5 times renorm.cu's time (n = 521, 1 / 31 angles: 4.2 / 6.8 ms
+//   against 1.2 / 3.7).
 constexpr int kWMax = 16;      // panel width the scratch is sized for
 constexpr int kUpdCols = 128;  // trailing columns per update block
 
 struct GJScratch {
-  int* piv;   // nang x kW
+  int* piv;   // nang x 2 kW
   cd* W1;     // nang x kW x kW
-  cd* L2;     // nang x n x kW
+  cd* L2;     // nang x n x 2 kW (the shared-memory path uses nang x n x kW of it)
 };
 
+// Pivots and multipliers: 2 kW per angle (the row-per-thread path keeps the pivots
+// and E of two panels; the shared-memory path uses the first kW of each).
 size_t gj_scratch_bytes(int nang, int n) {
-  size_t b = (size_t)nang * kWMax * sizeof(int);
+  size_t b = (size_t)nang * 2 * kWMax * sizeof(int);
   b = (b + 255) & ~size_t(255);
   b += (size_t)nang * kWMax * kWMax * sizeof(cd);
   b = (b + 255) & ~size_t(255);
-  b += (size_t)nang * n * kWMax * sizeof(cd);
+  b += (size_t)nang * n * 2 * kWMax * sizeof(cd);
   return std::max(b, n <= kGjClusterMaxRows ? gj_cluster_scratch_bytes(nang, n) : 0) + 256;
 }
 
@@ -444,7 +451,7 @@ static GJScratch gj_carve(void* scratch, int nang, int n) {
   GJScratch s;
   char* p = reinterpret_cast<char*>(scratch);
   s.piv = reinterpret_cast<int*>(p);
-  size_t b = (size_t)nang * kWMax * sizeof(int);
+  size_t b = (size_t)nang * 2 * kWMax * sizeof(int);
   b = (b + 255) & ~size_t(255);
   s.W1 = reinterpret_cast<cd*>(p + b);
   b += (size_t)nang * kWMax * kWMax * sizeof(cd);
@@ -588,6 +595,113 @@ __global__ void k_gj_panel(const cd* __restrict__ Q, const int* __restrict__ fla
   }
 }
 
+// Panel step for n <= kPanelRowsMax rows, one row per thread: Gauss-Jordan
+// elimination of the panel columns in place, with the pivot rule of k_gj_panel.
+// Column step jj pivots, swaps rows col and p, scales the pivot row by r = 1/d and
+// eliminates the column from every other row i with the multiplier g = f_i r
+// (f_i the row's entry in column jj): x_k <- x_k - g u_k for the other columns,
+// and the freed slot jj takes -g.  After w steps the panel holds E with
+// E [B1; B_other] = [I; 0] over the pivot columns: its pivot rows are B1^{-1}, its
+// other rows -B_other B1^{-1}.  The trailing update is then, after the same row
+// swaps, C1' = E_pivot C1 for the pivot rows and C' = C + E_i C1 for the others.
+// One barrier per column: each warp publishes its best candidate row, and the
+// owner of row col publishes that row, before it.
+constexpr int kPanelRowsMax = kGjClusterMaxRows;
+template <bool kF, int kMaxT>
+__global__ void __launch_bounds__(kMaxT, 1)
+    k_gj_panel_rows(const cd* __restrict__ Q, const int* __restrict__ flag, int n, int ld, int c0,
+                    int w, int* __restrict__ piv, int pstride, cd* __restrict__ E, int estride,
+                    unsigned* status) {
+  static_assert(kWMax == 16, "one 16-column panel per thread row");
+  const int a = blockIdx.x;
+  if (flag && !flag[a]) return;
+  constexpr int kMaxWarps = kMaxT / 32;
+  __shared__ double cand_v[2][kMaxWarps];
+  __shared__ int cand_i[2][kMaxWarps];
+  __shared__ cd cand_row[2][kMaxWarps][kWMax];
+  __shared__ cd crow[2][kWMax];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
+  const unsigned full = 0xffffffffu;
+  cd x[kWMax];
+  {
+    const cd* A = Q + (size_t)a * n * ld + (size_t)min(tid, n - 1) * ld + c0;
+#pragma unroll
+    for (int k = 0; k < kWMax; ++k) x[k] = (tid < n && k < w) ? A[k] : cd{0.0, 0.0};
+  }
+  // a runtime loop over the columns (an unrolled one overflows the instruction
+  // cache); column jj of the row is picked by a select over the 16 registers
+  for (int jj = 0; jj < w; ++jj) {
+    const int col = c0 + jj, buf = jj & 1;
+    // ---- this warp's candidate: max |re|+|im| over rows >= col, lowest row on ties
+    cd xj = x[0];
+#pragma unroll
+    for (int k = 1; k < kWMax; ++k)
+      if (k == jj) xj = x[k];
+    const bool live = tid >= col && tid < n;
+    double best = live ? cabs1(xj) : -1.0;
+    int bi = live ? tid : n;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const double ov = __shfl_xor_sync(full, best, o);
+      const int oi = __shfl_xor_sync(full, bi, o);
+      if (ov > best || (ov == best && oi < bi)) {
+        best = ov;
+        bi = oi;
+      }
+    }
+    if (tid == bi) {
+#pragma unroll
+      for (int k = 0; k < kWMax; ++k) cand_row[buf][warp][k] = x[k];
+    }
+    if (lane == 0) {
+      cand_v[buf][warp] = best;
+      cand_i[buf][warp] = bi;
+    }
+    if (tid == col) {
+#pragma unroll
+      for (int k = 0; k < kWMax; ++k) crow[buf][k] = x[k];
+    }
+    __syncthreads();
+    // ---- the block's pivot among the warp candidates
+    best = (lane < nw) ? cand_v[buf][lane] : -1.0;
+    bi = (lane < nw) ? cand_i[buf][lane] : n;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const double ov = __shfl_xor_sync(full, best, o);
+      const int oi = __shfl_xor_sync(full, bi, o);
+      if (ov > best || (ov == best && oi < bi)) {
+        best = ov;
+        bi = oi;
+      }
+    }
+    const int p = __shfl_sync(full, bi, 0), pw = p >> 5;  // row p is thread p's
+    if (tid == 0) piv[a * pstride + jj] = p;
+    const cd* u = cand_row[buf][pw];  // the pivot row (old row p)
+    const cd d = u[jj];  // shared memory: a dynamic index is fine
+    if (d.x == 0.0 && d.y == 0.0 && tid == 0) atomicOr(status, kStatusZeroPivot);
+    const double dinv = 1.0 / (d.x * d.x + d.y * d.y);  // 1/d = conj(d) / |d|^2
+    const cd r = cd{d.x * dinv, -d.y * dinv};
+    if (tid == col) {
+#pragma unroll
+      for (int k = 0; k < kWMax; ++k) x[k] = (k == jj) ? r : u[k] * r;
+    } else {
+      if (tid == p) {  // row p now holds the old row col
+#pragma unroll
+        for (int k = 0; k < kWMax; ++k) x[k] = crow[buf][k];
+        xj = crow[buf][jj];
+      }
+      const cd g = xj * r;
+#pragma unroll
+      for (int k = 0; k < kWMax; ++k) x[k] = (k == jj) ? -g : gj_sub<kF>(x[k], g, u[k]);
+    }
+  }
+  if (tid < n) {
+    cd* e = E + ((size_t)a * n + tid) * estride;
+#pragma unroll
+    for (int k = 0; k < kWMax; ++k) e[k] = x[k];
+  }
+}
+
 // Each CTA owns kUpdCols of the remaining columns of one angle.
 // One thread per column of the trailing matrix (Q columns right of the panel,
 // then every P column), 128 columns per block: the column's pivot-row values C1
@@ -689,6 +803,250 @@ __global__ void __launch_bounds__(kUpdCols, 4) k_gj_update(cd* __restrict__ Q, c
   }
 }
 
+// Trailing update from a Gauss-Jordan step's E on the FP64 tensor path (fused
+// rounding).  For the kW pivot rows c0..c0+w-1 (w <= kW) the step is, after its
+// row swaps, C' = C + E C1 for every row (C = 0 for the pivot rows, whose E rows
+// are B1^{-1}): a complex GEMM with K = kW over the trailing columns.  The columns
+// come in two segments (Q right of the panel and P; or the 16 columns of another
+// step's E), each with its own base, row stride and angle stride.  The CTA owns
+// kMmaCols columns of one angle; after a common setup its four warps work
+// independently on 16-row strips (warp w: strips w, w+4, ...).  Per strip: m16n8k4
+// FP64 MMAs, four real MMAs per complex product, accumulators initialised from C;
+// the warp's E rows come through its own two cp.async buffers and the next strip's
+// C values are loaded into registers while the current strip's MMAs run.
+// Row swaps: warp 0 replays the step's swap sequence on the (at most 2 kW) touched
+// row positions, so every position knows which original row its value comes from;
+// C1 (the pivot rows after the swaps) and the values that end in touched rows
+// below the pivot block are read into shared memory before any row is written,
+// and a strip reads a touched row from that stash.
+constexpr int kMmaCols = 32;        // complex columns per CTA (4 n8 tiles)
+constexpr int kStrip = 16;          // rows per warp strip
+constexpr int kC1Str = kMmaCols + 2;
+template <int kW>
+struct MmaUpdSmem {
+  static constexpr int kEStr = kW + 4;  // complex entries per E row in shared memory
+  cd E[4][2][kStrip][kEStr];
+  cd C1[kW][kC1Str];
+  cd stash[kW][kMmaCols];
+  short rslot[kMaxBeams];
+  int tpos[2 * kW], tsrc[2 * kW];
+  int ntouched;
+};
+
+// Trailing columns of an update: segment 0 (n0 columns) then segment 1.  Element
+// (r, vc) of angle a is p + a * as + r * ld + vc (vc counted within its segment).
+struct GjCols {
+  cd* p0;
+  long long as0;
+  int ld0, n0;
+  cd* p1;
+  long long as1;
+  int ld1, n1;
+};
+
+// One work item: angle a, trailing columns vc0 .. vc0 + kMmaCols - 1.
+template <int kW>
+__device__ __forceinline__ void gj_update_mma_item(MmaUpdSmem<kW>& sm, const GjCols& cols, int n,
+                                                   int c0, int w, const int* __restrict__ pivs,
+                                                   int pstride, const cd* __restrict__ E,
+                                                   int estride, int a, int vc0) {
+  constexpr int kNi = kMmaCols / 8, kSlots = (2 * kW + 31) / 32;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  const int total = cols.n0 + cols.n1;
+  cd* const b0 = cols.p0 + (size_t)a * cols.as0;
+  cd* const b1 = cols.p1 + (size_t)a * cols.as1;
+  // element (r, vc) of this angle's trailing columns (vc < total)
+  auto at = [&](int r, int vc) -> cd* {
+    return vc < cols.n0 ? b0 + (size_t)r * cols.ld0 + vc
+                        : b1 + (size_t)r * cols.ld1 + (vc - cols.n0);
+  };
+  const cd* Ea = E + (size_t)a * n * estride;
+  const int* pa = pivs + (size_t)a * pstride;
+  for (int i = tid; i < n; i += 128) sm.rslot[i] = -1;
+  __syncthreads();
+  if (warp == 0) {
+    // entry q (lane q & 31, slot q >> 5) holds a touched position and the row its
+    // value comes from: entries 0..w-1 are the pivot block, later ones the pivot
+    // rows below it in order of first use
+    int pos[kSlots], src[kSlots], myp[kSlots];
+#pragma unroll
+    for (int e = 0; e < kSlots; ++e) {
+      const int q = lane + 32 * e;
+      pos[e] = q < w ? c0 + q : -1;
+      src[e] = pos[e];
+      myp[e] = q < w ? pa[q] : 0;
+    }
+    int nt = w;
+    for (int jj = 0; jj < w; ++jj) {
+      int r1 = 0;
+#pragma unroll
+      for (int e = 0; e < kSlots; ++e)
+        if ((jj >> 5) == e) r1 = __shfl_sync(0xffffffffu, myp[e], jj & 31);
+      int i1 = -1;
+#pragma unroll
+      for (int e = kSlots - 1; e >= 0; --e) {
+        const unsigned hit = __ballot_sync(0xffffffffu, pos[e] == r1);
+        if (hit) i1 = 32 * e + __ffs(hit) - 1;
+      }
+      if (i1 < 0) {
+        i1 = nt++;
+#pragma unroll
+        for (int e = 0; e < kSlots; ++e)
+          if (lane + 32 * e == i1) pos[e] = src[e] = r1;
+      }
+      int sj = 0, si = 0;
+#pragma unroll
+      for (int e = 0; e < kSlots; ++e) {
+        const int vj = __shfl_sync(0xffffffffu, src[e], jj & 31);
+        const int vi = __shfl_sync(0xffffffffu, src[e], i1 & 31);
+        if ((jj >> 5) == e) sj = vj;
+        if ((i1 >> 5) == e) si = vi;
+      }
+#pragma unroll
+      for (int e = 0; e < kSlots; ++e) {
+        if (lane + 32 * e == jj) src[e] = si;
+        if (lane + 32 * e == i1) src[e] = sj;
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < kSlots; ++e) {
+      const int q = lane + 32 * e;
+      if (q < 2 * kW) {
+        sm.tpos[q] = pos[e];
+        sm.tsrc[q] = src[e];
+      }
+      if (q >= w && q < nt) sm.rslot[pos[e]] = (short)(q - w);
+    }
+    if (lane == 0) sm.ntouched = nt;
+  }
+  __syncthreads();
+  {
+    const int nt = sm.ntouched;
+#pragma unroll
+    for (int it = 0; it < 2 * kW * kMmaCols / 128; ++it) {
+      const int e = tid + it * 128, q = e / kMmaCols, c = e % kMmaCols, vc = vc0 + c;
+      if (q < kW) {
+        sm.C1[q][c] = (q < w && vc < total) ? *at(sm.tsrc[q], vc) : cd{0.0, 0.0};
+      } else {  // stash slot sl: touched entry w + sl (rows below the pivot block)
+        const int sl = q - kW, te = w + sl;
+        if (te < nt) sm.stash[sl][c] = vc < total ? *at(sm.tsrc[te], vc) : cd{0.0, 0.0};
+      }
+    }
+  }
+  __syncthreads();
+  // this thread's 8 columns are vc0 + ni * 8 + 2t + j; addresses formed on use
+  const int vt = vc0 + 2 * t;
+  auto fetch_e = [&](int strip, int b) {
+#pragma unroll
+    for (int q = 0; q < kStrip * kW / 32; ++q) {
+      const int e = lane + q * 32, r = e / kW, k = e % kW, row = strip * kStrip + r;
+      const cd* src = Ea + (size_t)min(row, n - 1) * estride + k;
+      const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&sm.E[warp][b][r][k]);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src),
+                   "r"(row < n ? 16 : 0)
+                   : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  // C values of a strip in accumulator order (0 in the pivot rows, stash values in
+  // touched rows)
+  auto load_c = [&](int strip, double (&cr)[kNi][4], double (&ci)[kNi][4]) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int r = strip * kStrip + g + 8 * h;
+      const bool live = r < n && !(r >= c0 && r < c0 + w);
+      const int sl = live ? sm.rslot[r] : -1;
+#pragma unroll
+      for (int ni = 0; ni < kNi; ++ni)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const int vc = vt + ni * 8 + j;
+          cd v = cd{0.0, 0.0};
+          if (live && vc < total) v = sl >= 0 ? sm.stash[sl][ni * 8 + 2 * t + j] : *at(r, vc);
+          cr[ni][2 * h + j] = v.x;
+          ci[ni][2 * h + j] = v.y;
+        }
+    }
+  };
+  const int nstrips = ceil_div(n, kStrip);
+  double cr[kNi][4], ci[kNi][4];
+  if (warp < nstrips) {
+    fetch_e(warp, 0);
+    load_c(warp, cr, ci);
+  }
+  int b = 0;
+  for (int strip = warp; strip < nstrips; strip += 4, b ^= 1) {
+    const int nxt = strip + 4;
+    double nr[kNi][4], nim[kNi][4];
+    if (nxt < nstrips) {
+      fetch_e(nxt, b ^ 1);
+      load_c(nxt, nr, nim);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+    __syncwarp();
+#pragma unroll
+    for (int kk = 0; kk < kW / 4; ++kk) {
+      const cd a0 = sm.E[warp][b][g][kk * 4 + t];
+      const cd a1 = sm.E[warp][b][g + 8][kk * 4 + t];
+#pragma unroll
+      for (int ni = 0; ni < kNi; ++ni) {
+        const cd bf = sm.C1[kk * 4 + t][ni * 8 + g];
+        double* R = cr[ni];
+        double* I = ci[ni];
+        dmma(R[0], R[1], R[2], R[3], a0.x, a1.x, bf.x);
+        dmma(R[0], R[1], R[2], R[3], -a0.y, -a1.y, bf.y);
+        dmma(I[0], I[1], I[2], I[3], a0.x, a1.x, bf.y);
+        dmma(I[0], I[1], I[2], I[3], a0.y, a1.y, bf.x);
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int r = strip * kStrip + g + 8 * h;
+      if (r < n) {
+#pragma unroll
+        for (int ni = 0; ni < kNi; ++ni)
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            const int vc = vt + ni * 8 + j;
+            if (vc < total) *at(r, vc) = cd{cr[ni][2 * h + j], ci[ni][2 * h + j]};
+          }
+      }
+    }
+    __syncwarp();  // the next fetch reuses this strip's buffer
+    if (nxt < nstrips) {
+#pragma unroll
+      for (int ni = 0; ni < kNi; ++ni)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          cr[ni][e] = nr[ni][e];
+          ci[ni][e] = nim[ni][e];
+        }
+    }
+  }
+}
+
+// Grid-stride over the (angle, column tile) items, so the last wave of a launch is
+// not left partly empty.
+template <int kW>
+__global__ void __launch_bounds__(128, kW == 16 ? 3 : 2)
+    k_gj_update_mma(GjCols cols, const int* __restrict__ flag, int n, int c0, int w,
+                    const int* __restrict__ pivs, int pstride, const cd* __restrict__ E,
+                    int estride, int nang) {
+  extern __shared__ __align__(16) unsigned char mma_dyn[];
+  MmaUpdSmem<kW>& sm = *reinterpret_cast<MmaUpdSmem<kW>*>(mma_dyn);
+  const int tiles = ceil_div(cols.n0 + cols.n1, kMmaCols);
+  for (int item = blockIdx.x; item < tiles * nang; item += gridDim.x) {
+    const int a = item / tiles;
+    if (flag && !flag[a]) continue;
+    gj_update_mma_item<kW>(sm, cols, n, c0, w, pivs, pstride, E, estride, a,
+                           (item - a * tiles) * kMmaCols);
+    __syncthreads();  // the next item reuses the shared memory
+  }
+}
+
 template <int kW, bool kF>
 static int gauss_jordan_smem(cd* Q, cd* P, const int* flag, int nang, int n, int ld,
                               const GJScratch& sc, unsigned* status, cudaStream_t st) {
@@ -705,16 +1063,105 @@ static int gauss_jordan_smem(cd* Q, cd* P, const int* flag, int nang, int n, int
   return 2 * ceil_div(n, kW);
 }
 
+static int gj_sm_count() {
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms > 0 ? sms : 148;
+}
+
+// The row-per-thread path, n <= 640: the row-per-thread panel (fused or product-first
+// complex arithmetic) and the trailing update on the FP64 tensor path.  The split
+// forms take 32 pivot columns per trailing update.  For columns c0..c0+31: the panel on the first 16
+// (E_a), a rank-16 update of the next 16 columns only, the panel on those (E_b),
+// the second step applied to E_a's 16 columns (so that [E_a | E_b] is the E of a
+// 32-column Gauss-Jordan step: the in-place elimination of the second half would
+// have updated the first half's slots), then one rank-32 update of every other
+// trailing column with the 32 row swaps in order.  The last panel of fewer than
+// 17 columns takes one rank-16 step.  E and the pivots live in the scratch's
+// 32-column blocks (row stride 32).
+template <bool kF>
+static int gauss_jordan_rows(cd* Q, cd* P, const int* flag, int nang, int n, int ld,
+                              const GJScratch& sc, unsigned* status, cudaStream_t st) {
+  static SmemOptIn attr16, attr32;
+  attr16.ensure((const void*)k_gj_update_mma<16>, sizeof(MmaUpdSmem<16>));
+  attr32.ensure((const void*)k_gj_update_mma<32>, sizeof(MmaUpdSmem<32>));
+  const int threads = round_up(n, 32), sms = gj_sm_count();
+  int launches = 0;
+  constexpr int kP = 2 * kWMax;  // pivots and E columns per angle in the scratch
+  const long long qa = (long long)n * ld, ea = (long long)n * kP;
+  auto panel = [&](int c, int w, int poff) {
+    ++launches;
+    int* pv = sc.piv + poff;
+    cd* E = sc.L2 + poff;
+    if (threads <= 256)
+      k_gj_panel_rows<kF, 256><<<nang, threads, 0, st>>>(Q, flag, n, ld, c, w, pv, kP, E, kP,
+                                                         status);
+    else if (threads <= 544)
+      k_gj_panel_rows<kF, 544><<<nang, threads, 0, st>>>(Q, flag, n, ld, c, w, pv, kP, E, kP,
+                                                         status);
+    else
+      k_gj_panel_rows<kF, kPanelRowsMax><<<nang, threads, 0, st>>>(Q, flag, n, ld, c, w, pv, kP,
+                                                                   E, kP, status);
+  };
+  auto update16 = [&](const GjCols& cols, int c, int w, int poff) {
+    const int items = ceil_div(cols.n0 + cols.n1, kMmaCols) * nang;
+    if (items == 0) return;
+    ++launches;
+    k_gj_update_mma<16><<<std::min(items, 3 * sms), 128, sizeof(MmaUpdSmem<16>), st>>>(
+        cols, flag, n, c, w, sc.piv + poff, kP, sc.L2 + poff, kP, nang);
+  };
+  if (!kF) {
+    // the FP64 form: rank-16 steps throughout (its parity against the reference's
+    // test521 sp6 0.68 output, 2e-9, holds with this blocking and not with the
+    // rank-32 one, 2.5e-9)
+    for (int c0 = 0; c0 < n; c0 += kWMax) {
+      const int w = std::min(kWMax, n - c0);
+      panel(c0, w, 0);
+      update16(GjCols{Q + c0 + w, qa, ld, n - c0 - w, P, qa, ld, n}, c0, w, 0);
+    }
+    return launches;
+  }
+  for (int c0 = 0; c0 < n;) {
+    const int rem = n - c0;
+    if (rem <= kWMax) {  // one rank-16 step: Q right of the panel (none) and P
+      panel(c0, rem, 0);
+      update16(GjCols{Q + c0 + rem, qa, ld, 0, P, qa, ld, n}, c0, rem, 0);
+      break;
+    }
+    const int wb = std::min(kWMax, rem - kWMax), w = kWMax + wb;
+    panel(c0, kWMax, 0);
+    // step a on the next panel's columns only
+    update16(GjCols{Q + c0 + kWMax, qa, ld, wb, P, qa, ld, 0}, c0, kWMax, 0);
+    panel(c0 + kWMax, wb, kWMax);
+    // step b on E_a's 16 columns
+    update16(GjCols{sc.L2, ea, kP, kWMax, P, qa, ld, 0}, c0 + kWMax, wb, kWMax);
+    // both steps on every other trailing column
+    const GjCols rest{Q + c0 + w, qa, ld, n - c0 - w, P, qa, ld, n};
+    const int items = ceil_div(rest.n0 + rest.n1, kMmaCols) * nang;
+    k_gj_update_mma<32><<<std::min(items, 2 * sms), 128, sizeof(MmaUpdSmem<32>), st>>>(
+        rest, flag, n, c0, w, sc.piv, kP, sc.L2, kP, nang);
+    ++launches;
+    c0 += w;
+  }
+  return launches;
+}
+
 int launch_gauss_jordan(cd* Q, cd* P, const int* flag, int nang, int n, int ld, void* scratch,
                         unsigned* status, cudaStream_t st, int arith) {
-  if (arith != kGjProductFirst && n <= kGjClusterMaxRows)
+  const bool small = n <= kGjClusterMaxRows;
+  if (small && (arith == kGjFp64 || arith == kGjFused))
     return launch_gj_cluster(Q, P, flag, nang, n, ld, scratch, status, st);
   const GJScratch sc = gj_carve(scratch, nang, n);
-  if (arith == kGjProductFirst)
-    return gauss_jordan_smem<kWMax, false>(Q, P, flag, nang, n, ld, sc, status, st);
-  const int launches = arith == kGjFused
-                           ? gauss_jordan_smem<kWMax, true>(Q, P, flag, nang, n, ld, sc, status, st)
-                           : gauss_jordan_smem<kWMax, false>(Q, P, flag, nang, n, ld, sc, status, st);
+  const bool fused = arith == kGjFused || arith == kGjFusedRows;
+  int launches;
+  if (small && arith != kGjProductFirst)
+    launches = fused ? gauss_jordan_rows<true>(Q, P, flag, nang, n, ld, sc, status, st)
+                     : gauss_jordan_rows<false>(Q, P, flag, nang, n, ld, sc, status, st);
+  else
+    launches = fused ? gauss_jordan_smem<kWMax, true>(Q, P, flag, nang, n, ld, sc, status, st)
+                     : gauss_jordan_smem<kWMax, false>(Q, P, flag, nang, n, ld, sc, status, st);
+  if (arith == kGjProductFirst) return launches;
   launch_set_identity(Q, flag, nang, n, ld, st);
   return launches + 1;
 }

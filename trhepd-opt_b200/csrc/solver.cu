@@ -228,6 +228,7 @@ struct RunState {
   int nprob = 1;             // stacked problems (see trhepd_problem::nprob)
   const TableEntry* const* tables = nullptr;
   StackedRows sr{};          // rows and stage-matrix stride per stacked problem
+  int gj = kGjFp64, gj_edge = kGjFp64;  // renormalisations; boundary transforms
   bool conv = false;         // stage products as convolutions (convolve.h)
   ConvStages cs{};           // their constant arguments
   const int* centry = nullptr;
@@ -265,6 +266,7 @@ struct trhepd_problem {
   DevBuf ccell, cmask, centry, cD;
   Integrator I{};
   double dz = 0, kappa_max = 0;
+  double gamma_max = 0, gamma_rms = 0;  // |gamma| over all beams and angles
   int ncol = 0;
   DevBuf table, pair, gam, D, F, wnsga2, f2, dang, conv;
   std::vector<double> angle_deg;
@@ -384,7 +386,7 @@ void prepare(trhepd_context* C, const SolveArgs& A, trhepd_problem& Pb) {
   if (sum != n) throw std::invalid_argument("sum(nbg) != nb");
   for (int i = 0; i < n; ++i)
     if (A.iord[i] < 1 || A.iord[i] > n) throw std::invalid_argument("iord out of range");
-  double kappa_max = 0.0;
+  double kappa_max = 0.0, gamma2_max = 0.0, gamma2_sum = 0.0;
   for (int t = 0; t < nang; ++t) {
     int irep1 = t / nrep2, irep2 = t % nrep2;
     double ga, az;
@@ -407,10 +409,14 @@ void prepare(trhepd_context* C, const SolveArgs& A, trhepd_problem& Pb) {
       cd g2 = g * g;
       Dm[(size_t)t * ld + i] = cd{-g2.x, g2.y};  // -conj(g^2)
       if (s < 0) kappa_max = std::max(kappa_max, std::sqrt(-s));
+      gamma2_max = std::max(gamma2_max, std::abs(s));
+      gamma2_sum += std::abs(s);
     }
     Pb.angle_deg[t] = (ng_outer ? ga : az) * 180.0 / 3.141592654;
   }
   Pb.kappa_max = kappa_max;
+  Pb.gamma_max = std::sqrt(gamma2_max);
+  Pb.gamma_rms = std::sqrt(gamma2_sum / ((double)nang * n));
   Pb.nb0 = 0;
   for (int i = 0; i < n; ++i)
     if (A.ih[i] == 0 && A.ik[i] == 0) Pb.nb0 = i;
@@ -454,6 +460,21 @@ Workspace context_workspace(trhepd_context* C) {
           &C->spec};
 }
 
+// Solves that amplify a change of rounding keep one sequence of operations: dense or digit
+// stage products and the row-swapping elimination (kGj*Rows, kGjProductFirst at the
+// boundaries), whose results other sequences reproduce to less than 1e-9 only here:
+// * RK4 (int_method 7 and 8).  It damps propagating beams and, beyond |gamma| dz = 2.8, is
+//   unstable; what the eliminations then divide by amplifies a rounding 1e3 (|gamma| dz =
+//   1.5) to 1e9 times (2.1: 3e-8 of the curve at n = 40, 2.6: 3e-6 at n = 351) and the
+//   digits' truncation to 2e-8 at |gamma| dz = 1.8, n = 17.
+// * the split forms on coarse slices: the digits' truncation (2e-12 per product) shows as
+//   1e-11 of the curve at rms |gamma| dz = 6, 1e-10 at 7.5 and up to 2e-8 at 9, and falls
+//   differently after another elimination.
+bool rounding_amplified(const trhepd_problem& Pb, bool split) {
+  if (Pb.I.family == kRk4) return split || Pb.gamma_max * Pb.dz > 1.5;
+  return split && Pb.gamma_rms * Pb.dz > 7.5;
+}
+
 // Whether the stage products of a solve are convolutions over the beam grid.  Against the
 // dense FP64 products they pay wherever conv_grid returns a grid (n = 521, 16 angles: 0.68
 // -> 0.17 ms per stage; n = 95, 61 angles: 56 -> 14.5 us).  Against the digit products (5
@@ -463,8 +484,12 @@ Workspace context_workspace(trhepd_context* C) {
 // m = 25: 102 against 157) nor with fewer slices (n = 521, 4 slices: 330).
 bool use_convolution(const trhepd_context* C, const trhepd_problem& Pb, bool split) {
   const int m = Pb.grid.m;
-  if (!m || Pb.I.family > kRk4) return false;
-  if (!split || m <= 16) return true;
+  if (!m || Pb.I.family > kRk4 || rounding_amplified(Pb, split)) return false;
+  if (!split) return true;
+  // the split forms' results stay those of the digits: their truncation, which the
+  // convolution does not have, is below 1e-11 of the curve up to here and 4e-9 at 8
+  if (Pb.gamma_rms * Pb.dz > 3.0) return false;
+  if (m <= 16) return true;
   return C->split_slices >= 5 && m <= 27 && (double)Pb.n >= 0.7 * m * m;
 }
 
@@ -487,6 +512,12 @@ void begin_run(trhepd_context* C, trhepd_problem& Pb, int precision, int nprod_m
   R.sbytes = (size_t)nang * n * ld * sizeof(cd);
   R.split = precision == TRHEPD_SPLIT_BF16 || precision == TRHEPD_SPLIT_INT8;
   R.conv = use_convolution(C, Pb, R.split);
+  if (rounding_amplified(Pb, R.split)) {
+    R.gj = R.split ? kGjFusedRows : kGjFp64Rows;
+    R.gj_edge = kGjProductFirst;
+  } else {
+    R.gj = R.gj_edge = R.split ? kGjFused : kGjFp64;
+  }
   R.Q = (cd*)W.Q0->ensure(R.sbytes);
   if (!R.conv) R.Qn = (cd*)W.Q1->ensure(R.sbytes);  // the dense products' second Q
   R.P = (cd*)W.P->ensure(R.sbytes);
@@ -558,9 +589,13 @@ void begin_run(trhepd_context* C, trhepd_problem& Pb, int precision, int nprod_m
   // invstransh: Q = I + F^H, P = I - F^H; P <- Q^{-1} P; P <- i P conj(G); Q = I
   launch_invstransh_build(Pb.F.as<cd>(), R.Q, R.P, nang, n, ld, st);
   R.launches += launch_gauss_jordan(R.Q, R.P, nullptr, nang, n, ld, R.gjs, R.status, st,
-                                    R.split ? kGjFused : kGjFp64);
+                                    R.gj_edge);
   launch_invstransh_finish(R.P, R.gam, nang, n, ld, st);
   R.launches += 2;
+  if (R.gj_edge == kGjProductFirst) {  // leaves Q as it is
+    launch_set_identity(R.Q, nullptr, nang, n, ld, st);
+    R.launches += 1;
+  }
   if (C->renorm_policy == 1) {
     double kap = Pb.kappa_max + 1.0;
     R.interval = std::max(1, (int)std::floor(C->renorm_tau / (kap * Pb.dz)));
@@ -671,13 +706,13 @@ void renormalise_launch(trhepd_context* C, RunState& R, bool last, int l, bool e
   if (C->renorm_policy == 0 && !every_slice) {
     launch_cond_est(R.Q, R.nang, R.n, R.ld, last ? 1 : 0, R.flags, R.dval, R.st);
     const int k = launch_gauss_jordan(R.Q, R.P, R.flags, R.nang, R.n, R.ld, R.gjs, R.status,
-                                      R.st, R.split ? kGjFused : kGjFp64);
+                                      R.st, R.gj);
     R.launches += 1 + k;
     R.gj_launches += k;
     if (!last) ++R.renorms;  // upper bound; per-angle decisions stay on the device
   } else if (last || every_slice || (l % R.interval) == 0) {
     const int k = launch_gauss_jordan(R.Q, R.P, nullptr, R.nang, R.n, R.ld, R.gjs, R.status,
-                                      R.st, R.split ? kGjFused : kGjFp64);
+                                      R.st, R.gj);
     R.launches += k;
     R.gj_launches += k;
     if (!last) ++R.renorms;
@@ -693,7 +728,7 @@ void finish_device(trhepd_context* C, trhepd_problem& Pb, RunState& R) {
   else
     launch_stransh_build(R.Q, R.P, R.gam, nang, n, ld, st);
   R.launches += launch_gauss_jordan(R.Q, R.P, nullptr, nang, n, ld, R.gjs, R.status, st,
-                                    R.split ? kGjFused : kGjFp64);
+                                    R.gj_edge);
   launch_check_finite(R.P, (size_t)nang * n * ld, R.status, st);
   launch_intensities(R.P, R.gam, Pb.wnsga2.as<double>(), nang, n, ld, Pb.nb0,
                      Pb.f2.as<double>(), st);
@@ -872,7 +907,8 @@ void run_lf(trhepd_context* C, trhepd_problem& Pb, int precision, RunState& R) {
 void run_rk4(trhepd_context* C, trhepd_problem& Pb, int precision, RunState& R) {
   const double dz = Pb.dz;
   begin_run(C, Pb, precision, 4 * Pb.ns, R, context_workspace(C));
-  if (!R.split && !Pb.I.gs && Pb.n <= C->fused_max_n && fused_rk4_fits(Pb.n, Pb.nv)) {
+  if (!Pb.I.gs && !rounding_amplified(Pb, R.split) && Pb.n <= C->fused_max_n &&
+      fused_rk4_fits(Pb.n, Pb.nv)) {
     fused_launch(C, Pb, R, launch_fused_rk4);
     R.products += 4L * R.ns;
     R.renorms += (C->renorm_policy == 1) ? (R.ns - 1) / R.interval : R.ns - 1;
@@ -1122,12 +1158,16 @@ void run_checked(trhepd_context* C, trhepd_problem& Pb, int precision) {
 
 // Problems that can be integrated as one stacked solve: same beams and beam-pair
 // map, slice count and thickness, integrator and angle count (the candidates of
-// one base structure).  Their angles are stacked row-wise; each row tile of the
-// stage product reads its own problem's stage matrix.
-bool stackable(const trhepd_problem& a, const trhepd_problem& b) {
-  return a.n == b.n && a.ns == b.ns && a.dz == b.dz && a.int_method == b.int_method &&
-         a.nang == b.nang && a.nv == b.nv && a.ncol == b.ncol && a.nb0 == b.nb0 &&
-         a.grid.m == b.grid.m && a.grid.cell == b.grid.cell && a.pair_host == b.pair_host;
+// one base structure), which each on its own would take the same path.  Their angles
+// are stacked row-wise; each row tile of the stage product reads its own problem's
+// stage matrix.
+bool stackable(const trhepd_context* C, const trhepd_problem& a, const trhepd_problem& b,
+               bool split) {
+  return rounding_amplified(a, split) == rounding_amplified(b, split) &&
+         use_convolution(C, a, split) == use_convolution(C, b, split) && a.n == b.n &&
+         a.ns == b.ns && a.dz == b.dz && a.int_method == b.int_method && a.nang == b.nang &&
+         a.nv == b.nv && a.ncol == b.ncol && a.nb0 == b.nb0 && a.grid.m == b.grid.m &&
+         a.grid.cell == b.grid.cell && a.pair_host == b.pair_host;
 }
 
 // One integration of a stacked group; the intensities go back to each problem.
@@ -1149,7 +1189,11 @@ void solve_stacked(trhepd_context* C, const std::vector<trhepd_problem*>& g, int
   M.nrep2 = p0.nrep2;
   M.nang = k * na;
   M.nprob = k;
-  for (const trhepd_problem* p : g) M.kappa_max = std::max(M.kappa_max, p->kappa_max);
+  for (const trhepd_problem* p : g) {
+    M.kappa_max = std::max(M.kappa_max, p->kappa_max);
+    M.gamma_max = std::max(M.gamma_max, p->gamma_max);
+    M.gamma_rms = std::max(M.gamma_rms, p->gamma_rms);
+  }
   M.pair.p = p0.pair.p;    // borrowed (shared beam-pair map)
   M.table.p = p0.table.p;  // borrowed (the tables array holds every problem's)
   M.grid = p0.grid;
@@ -1268,7 +1312,7 @@ void batch_solve(trhepd_context* C, trhepd_problem* const* probs, int count, int
       done[q] = true;
       if (stack_ok && rest[q]->I.family == kRkn && rest[q]->n >= 2)
         for (size_t r = q + 1; r < rest.size(); ++r)
-          if (!done[r] && stackable(*rest[q], *rest[r]) &&
+          if (!done[r] && stackable(C, *rest[q], *rest[r], precision != TRHEPD_FP64) &&
               (long long)(grp.size() + 1) * rest[q]->nang * rest[q]->n <= (1 << 22)) {
             grp.push_back(rest[r]);
             done[r] = true;
