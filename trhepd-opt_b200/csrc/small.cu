@@ -37,6 +37,7 @@ namespace fused {
 
 constexpr int kThreads = 128;
 constexpr int kTabBufs = 4;  // table columns in flight where shared memory allows
+constexpr int kMaxEntries = (1 << 14) - 1;  // the fragment codes have 15 bits of position
 
 // RT row tiles; GW column groups per warp.  kRk4: the classical RK4 steps of rk4_int
 // (surf_rk.f90:27-91) instead of the RKN kicks: Q, P, the stage point's Q and the two
@@ -57,6 +58,8 @@ struct Cfg {
   // RK4 sum: it is dead at the end of a slice), and the fragment codes (8 bytes per lane and
   // k step)
   static constexpr size_t extra = kRk4 ? (size_t)3 * NP * STR : (size_t)16 * STR;
+  // beyond 48 beams a single column buffer also holds the pivot rows
+  static constexpr bool SHARE = RT > 3 && !kRk4;
   static constexpr size_t elems =
       (size_t)(QB + (PREG ? 0 : 1)) * NP * STR + extra + KS * kThreads / 2;
 };
@@ -108,12 +111,14 @@ __global__ void __launch_bounds__(kThreads, Cfg<RT, GW, kRk4>::MINB)
   cd* Qs = reinterpret_cast<cd*>(smem_raw);             // the current Q
   cd* Qo = Qs + (C::QB - 1) * NP * STR;                 // the other (the same for QB = 1)
   cd* const Ps = Qs + C::QB * NP * STR;                 // PREG = false only
-  cd* const c1s = Ps + (C::PREG ? 0 : NP * STR);        // 16 pivot rows
-  cd* const SQ = c1s;                                   // kRk4 only, as the next two
+  cd* const SQ = Ps + (C::PREG ? 0 : NP * STR);         // kRk4 only, as the next two
   cd* const SP = SQ + NP * STR;
   cd* const Qt = SP + NP * STR;
-  uint2* const codes = reinterpret_cast<uint2*>(c1s + C::extra);  // [KS][kThreads]
-  cd* const tab = c1s + C::extra + C::KS * kThreads / 2;          // [nbuf][tab_stride]
+  const bool one = C::SHARE && nbuf == 1;  // the pivot rows share the only column buffer
+  cd* const codes_at = SQ + (one ? 0 : C::extra);
+  uint2* const codes = reinterpret_cast<uint2*>(codes_at);  // [KS][kThreads]
+  cd* const tab = codes_at + C::KS * kThreads / 2;          // [nbuf][tab_stride]
+  cd* const c1s = one ? tab : SQ;                           // 16 pivot rows
   __shared__ double csum[kThreads];
   __shared__ double red_d[2][4];
   __shared__ unsigned keys[2][32];
@@ -265,15 +270,16 @@ __global__ void __launch_bounds__(kThreads, Cfg<RT, GW, kRk4>::MINB)
       mma(af[1], bf[1]);
     }
   };
-  // P += cb (Q V + Q o D), Q <- Q + ca P with the next table column; ends without a barrier
-  auto stage = [&](double cb, double ca) {
+  // P += cb (Q V + Q o D), Q <- Q + ca P with the next table column; ends without a barrier.
+  // hold: an elimination may follow, a column that shares its buffer is fetched after it.
+  auto stage = [&](double cb, double ca, bool hold) {
     const cd* tc = tab + out * tab_stride;
     arrived();
     __syncthreads();  // Q is there too
     if (nbuf > 1) fetch();
     product(Qs, tc);
     if (C::QB == 1 || nbuf == 1) __syncthreads();  // every read of Q and the column done
-    if (nbuf == 1) fetch();
+    if (nbuf == 1 && !(one && hold)) fetch();
 #pragma unroll
     for (int i = 0; i < TW; ++i)
 #pragma unroll
@@ -517,6 +523,14 @@ __global__ void __launch_bounds__(kThreads, Cfg<RT, GW, kRk4>::MINB)
       __syncthreads();
       gauss_jordan();
     }
+    if (one) {
+      if (renorm) {  // the pivot rows may have passed over the zero entry
+        if (tid < 2) tab[2 * nv + tid] = cd{0.0, 0.0};
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // before the copy's writes
+        __syncthreads();
+      }
+      fetch();
+    }
   };
   if constexpr (kRk4) {
     // stage j: weight of k_j in the sum, step to the next stage point; the middle column
@@ -571,12 +585,12 @@ __global__ void __launch_bounds__(kThreads, Cfg<RT, GW, kRk4>::MINB)
       for (int k = 1; k <= s; ++k) {
         // k == 1 merges the end-of-slice half kick of slice l-1 with the first kick
         const double cb = (k == 1) ? (l == 1 ? 1.0 : 2.0) * L.bab[0] * dz : L.bab[2 * k - 2] * dz;
-        stage(cb, L.bab[2 * k - 1] * dz);
+        stage(cb, L.bab[2 * k - 1] * dz, k == s);
       }
       end_of_slice(l);
     }
     // final half kick with Q = I: P += b1 dz M(end)
-    stage(L.bab[0] * dz, 0.0);
+    stage(L.bab[0] * dz, 0.0, false);
   }
   if (tid == 0 && dead)  // copies still on their way (as long as they may take)
     while (consumed < issued) {
@@ -605,27 +619,41 @@ __global__ void __launch_bounds__(kThreads, Cfg<RT, GW, kRk4>::MINB)
 
 // Shared memory of a launch: four column buffers where they leave the CTAs per SM the
 // registers allow, else two or one (a column's copy takes longer than a stage of a small
-// problem).
+// problem).  A single buffer is longer than the 16 pivot rows that share it: so every set
+// of 64 beams fits (2017 entries, 31 angles: 51 ms; 156 with a launch per stage, 95 with
+// gathered matrices in place of the table column).
 template <int RT, int GW, bool kRk4>
-int buffers(int stride, size_t& smem) {
+constexpr int buffers(int stride, size_t& smem) {
   using C = Cfg<RT, GW, kRk4>;
-  auto bytes = [&](int b) { return (C::elems + (size_t)b * stride) * sizeof(cd); };
+  auto bytes = [&](int b) {
+    return (C::elems - (b == 1 && C::SHARE ? C::extra : 0) + (size_t)b * stride) * sizeof(cd);
+  };
   int nbuf = bytes(kTabBufs) <= size_t(227 * 1024) / C::MINB - 4096 ? kTabBufs : 2;
   if (bytes(nbuf) > 224 * 1024) nbuf = 1;
   smem = bytes(nbuf);
   return smem <= 224 * 1024 ? nbuf : 0;
 }
+// Whether nv table entries a column fit; RK4 keeps a column through two stages.
+template <int RT, int GW, bool kRk4>
+constexpr bool fits(int nv) {
+  size_t smem = 0;
+  return nv >= 1 && nv <= kMaxEntries &&
+         buffers<RT, GW, kRk4>(2 * (nv + 1), smem) >= (kRk4 ? 2 : 1);
+}
+// the limits small.h states
+static_assert(fits<3, 3, false>(48 * 47 / 2 + 1));
+static_assert(fits<4, 4, false>(2303) && !fits<4, 4, false>(2304));
+static_assert(fits<3, 3, true>(271) && !fits<3, 3, true>(272));
 
+// A launch that fits.
 template <int RT, int GW, bool kRk4 = false>
-bool launch(const FusedLaunch& L, int nvmax, cudaStream_t st) {
+void launch(const FusedLaunch& L, int nvmax, cudaStream_t st) {
   static SmemOptIn attr;
   const int stride = 2 * (nvmax + 1);
   size_t smem = 0;
   const int nbuf = buffers<RT, GW, kRk4>(stride, smem);
-  if (nbuf < (kRk4 ? 2 : 1)) return false;  // RK4 keeps a column through two stages
   attr.ensure((const void*)k_fused_rkn<RT, GW, kRk4>, smem);
   k_fused_rkn<RT, GW, kRk4><<<L.total_ctas, kThreads, smem, st>>>(L, nbuf, stride);
-  return true;
 }
 
 }  // namespace fused
@@ -640,7 +668,7 @@ void check(const FusedLaunch& L, int& nmax, int& nvmax) {
   for (int q = 0; q < L.nprob; ++q) {
     const FusedProblem& a = L.p[q];
     if (a.n < 2 || a.n > kFusedMaxBeams || a.ns < 1 || a.interval < 1 || a.nang < 1 ||
-        a.first_cta != ctas || a.nv < 1 || a.nv > kFusedMaxEntries)
+        a.first_cta != ctas || a.nv < 1)
       throw std::invalid_argument("fused integration: unsupported problem");
     ctas += a.nang;
     nmax = std::max(nmax, a.n);
@@ -650,26 +678,33 @@ void check(const FusedLaunch& L, int& nmax, int& nvmax) {
 }
 }  // namespace
 
+bool fused_rkn_fits(int n, int nv) {
+  return n >= 2 && n <= kFusedMaxBeams &&
+         (n <= 16   ? fused::fits<1, 1, false>(nv)
+          : n <= 24 ? fused::fits<2, 3, false>(nv)
+          : n <= 32 ? fused::fits<2, 4, false>(nv)
+          : n <= 48 ? fused::fits<3, 3, false>(nv)
+                    : fused::fits<4, 4, false>(nv));
+}
+
 int launch_fused_rkn(const FusedLaunch& L, cudaStream_t st) {
   int nmax = 0, nvmax = 0;
   check(L, nmax, nvmax);
-  const bool ok = nmax <= 16   ? fused::launch<1, 1>(L, nvmax, st)
-                  : nmax <= 24 ? fused::launch<2, 3>(L, nvmax, st)
-                  : nmax <= 32 ? fused::launch<2, 4>(L, nvmax, st)
-                  : nmax <= 48 ? fused::launch<3, 3>(L, nvmax, st)
-                               : fused::launch<4, 4>(L, nvmax, st);
-  if (!ok) throw std::invalid_argument("fused integration: shared memory");
+  if (!fused_rkn_fits(nmax, nvmax)) throw std::invalid_argument("fused integration: shared memory");
+  if (nmax <= 16) fused::launch<1, 1>(L, nvmax, st);
+  else if (nmax <= 24) fused::launch<2, 3>(L, nvmax, st);
+  else if (nmax <= 32) fused::launch<2, 4>(L, nvmax, st);
+  else if (nmax <= 48) fused::launch<3, 3>(L, nvmax, st);
+  else fused::launch<4, 4>(L, nvmax, st);
   return 1;
 }
 
 bool fused_rk4_fits(int n, int nv) {
-  size_t smem = 0;
-  const int stride = 2 * (nv + 1);
-  return n >= 2 && n <= kFusedRk4MaxBeams && nv >= 1 && nv <= kFusedMaxEntries &&
-         (n <= 16   ? fused::buffers<1, 1, true>(stride, smem)
-          : n <= 24 ? fused::buffers<2, 3, true>(stride, smem)
-          : n <= 32 ? fused::buffers<2, 4, true>(stride, smem)
-                    : fused::buffers<3, 3, true>(stride, smem)) >= 2;
+  return n >= 2 && n <= kFusedRk4MaxBeams &&
+         (n <= 16   ? fused::fits<1, 1, true>(nv)
+          : n <= 24 ? fused::fits<2, 3, true>(nv)
+          : n <= 32 ? fused::fits<2, 4, true>(nv)
+                    : fused::fits<3, 3, true>(nv));
 }
 
 int launch_fused_rk4(const FusedLaunch& L, cudaStream_t st) {

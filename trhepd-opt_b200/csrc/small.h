@@ -9,10 +9,13 @@
 namespace trhepd {
 
 // Largest beam count of the fused kernel: Q, P, the pivot rows and one table column of an
-// angle (64 x 68 complex each of the first two) fit the 227 KB of shared memory.
+// angle (64 x 68 complex each of the first two) share the 227 KB of shared memory.
 constexpr int kFusedMaxBeams = 64;
-// Table entries per stage column it takes: every beam difference of 64 beams and more.
-constexpr int kFusedMaxEntries = 2100;
+// Whether a launch whose largest problem has n beams and whose longest stage column has nv
+// entries fits: up to 48 beams with every difference of theirs, 49 to 64 beams with at most
+// 2303 entries (64 beams have up to 2017 differences; the bulk file's list may add some of
+// them in the other order).
+bool fused_rkn_fits(int n, int nv);
 
 // One problem of a fused launch: its RKN integration (hp_int_spa,
 // surf_prkn.f90:278-330).  Q and P enter as the state after invstransh (Q = I)
@@ -41,12 +44,13 @@ struct FusedLaunch {
   FusedProblem p[kFusedMaxProblems];
 };
 
-// Launch the fused integration (one CTA per angle of every problem).  Returns
-// the number of kernels launched.
+// Launch the fused integration (one CTA per angle of every problem) of problems that
+// fit together.  Returns the number of kernels launched.
 int launch_fused_rkn(const FusedLaunch& L, cudaStream_t st);
 
 // The same for classical RK4 (rk4_int, surf_rk.f90:27-91; L.s = 2 table columns per slice,
-// L.bab unused).  Its five arrays fit one SM up to 48 beams and, there, 278 table entries.
+// L.bab unused).  Its five arrays fit one SM up to 48 beams and, from 33 beams on, 271
+// table entries.
 constexpr int kFusedRk4MaxBeams = 48;
 bool fused_rk4_fits(int n, int nv);
 int launch_fused_rk4(const FusedLaunch& L, cudaStream_t st);

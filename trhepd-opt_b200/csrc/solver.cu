@@ -819,8 +819,7 @@ void run_rkn(trhepd_context* C, trhepd_problem& Pb, int precision, RunState& R) 
   const double dz = Pb.dz;
   begin_run(C, Pb, precision, I.s * Pb.ns, R, context_workspace(C));
   const bool every_slice = (Pb.n == 1 && Pb.int_method == 6);  // hp_int_spa1d renormalises each slice
-  if (!R.split && R.nprob == 1 && Pb.n >= 2 && Pb.n <= std::min(C->fused_max_n, kFusedMaxBeams) &&
-      Pb.nv <= kFusedMaxEntries) {
+  if (!R.split && R.nprob == 1 && Pb.n <= C->fused_max_n && fused_rkn_fits(Pb.n, Pb.nv)) {
     fused_launch(C, Pb, R, launch_fused_rkn);
     R.products += (long)I.s * R.ns - 1;
     R.renorms += (C->renorm_policy == 1) ? (R.ns - 1) / R.interval : R.ns - 1;
@@ -1241,21 +1240,34 @@ void solve_stacked(trhepd_context* C, const std::vector<trhepd_problem*>& g, int
 // Problems solved together (no counterpart in the reference, whose driver solves
 // one structure at a time).  Problems the fused kernel takes (RKN, 2 <= n <= the
 // fused limit) are integrated by shared launches, each in its own buffers: one
-// launch per integrator and kFusedMaxProblems problems, whatever their beam
-// counts, slice counts and angle grids; the boundary kernels of each problem run
+// launch per integrator and kFusedMaxProblems problems that fit it together, whatever
+// their beam counts, slice counts and angle grids; the boundary kernels of each problem run
 // around it.  Other problems are solved one after another (graph replays from
 // their second solve on).  The split forms apply to those; fused problems are FP64.
 void batch_solve(trhepd_context* C, trhepd_problem* const* probs, int count, int precision) {
   cudaStream_t st = C->stream;
-  const int fmax = std::min(C->fused_max_n, kFusedMaxBeams);
-  std::vector<trhepd_problem*> fused[2], rest;  // by integrator: RKN-4 (s = 6), RKN-6 (s = 11)
+  // a fused launch: problems of one integrator that fit together
+  struct Group {
+    std::vector<trhepd_problem*> p;
+    int n = 0, nv = 0;  // the most beams and table entries
+  };
+  std::vector<Group> fused;
+  std::vector<trhepd_problem*> rest;
   for (int q = 0; q < count; ++q) {
     trhepd_problem* p = probs[q];
     if (!p) throw std::invalid_argument("null problem in batch");
-    if (p->I.family == kRkn && p->n >= 2 && p->n <= fmax && p->nv <= kFusedMaxEntries)
-      fused[p->I.s == 6 ? 0 : 1].push_back(p);
-    else
+    if (p->I.family != kRkn || p->n > C->fused_max_n || !fused_rkn_fits(p->n, p->nv)) {
       rest.push_back(p);
+      continue;
+    }
+    auto g = std::find_if(fused.begin(), fused.end(), [&](const Group& f) {
+      return f.p[0]->I.s == p->I.s && f.p.size() < (size_t)kFusedMaxProblems &&
+             fused_rkn_fits(std::max(f.n, p->n), std::max(f.nv, p->nv));
+    });
+    if (g == fused.end()) g = fused.insert(g, Group{});
+    g->p.push_back(p);
+    g->n = std::max(g->n, p->n);
+    g->nv = std::max(g->nv, p->nv);
   }
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   CK(cudaEventCreate(&e0));
@@ -1265,34 +1277,33 @@ void batch_solve(trhepd_context* C, trhepd_problem* const* probs, int count, int
   try {
     CK(cudaEventRecord(e0, st));
     static thread_local FusedLaunch L;
-    for (auto& group : fused)
-      for (size_t g0 = 0; g0 < group.size(); g0 += kFusedMaxProblems) {
-        const size_t g1 = std::min(group.size(), g0 + (size_t)kFusedMaxProblems);
-        std::vector<RunState> runs(g1 - g0);
-        const Integrator& I = group[g0]->I;
-        L.nprob = (int)(g1 - g0);
-        L.s = I.s;
-        L.policy = C->renorm_policy;
-        for (int q = 0; q < 2 * I.s + 1; ++q) L.bab[q] = I.bab[q];
-        int ctas = 0;
-        for (size_t q = g0; q < g1; ++q) {
-          RunState& R = runs[q - g0];
-          R.capturing = true;  // timing events belong to the batch
-          begin_run(C, *group[q], TRHEPD_FP64, 0, R, group[q]->own.view());
-          L.p[q - g0] = fused_problem(R, group[q]->dz, ctas);
-          ctas += R.nang;
-          products += (long)I.s * R.ns - 1;
-          renorms += (C->renorm_policy == 1) ? (R.ns - 1) / R.interval : R.ns - 1;
-        }
-        L.total_ctas = ctas;
-        launches += launch_fused_rkn(L, st);
-        for (size_t q = g0; q < g1; ++q) {
-          RunState& R = runs[q - g0];
-          finish_device(C, *group[q], R);
-          launches += R.launches;
-          statuses.push_back(R.status);
-        }
+    for (const Group& group : fused) {
+      std::vector<RunState> runs(group.p.size());
+      const Integrator& I = group.p[0]->I;
+      L.nprob = (int)group.p.size();
+      L.s = I.s;
+      L.policy = C->renorm_policy;
+      for (int q = 0; q < 2 * I.s + 1; ++q) L.bab[q] = I.bab[q];
+      int ctas = 0;
+      for (size_t q = 0; q < group.p.size(); ++q) {
+        trhepd_problem& p = *group.p[q];
+        RunState& R = runs[q];
+        R.capturing = true;  // timing events belong to the batch
+        begin_run(C, p, TRHEPD_FP64, 0, R, p.own.view());
+        L.p[q] = fused_problem(R, p.dz, ctas);
+        ctas += R.nang;
+        products += (long)I.s * R.ns - 1;
+        renorms += (C->renorm_policy == 1) ? (R.ns - 1) / R.interval : R.ns - 1;
       }
+      L.total_ctas = ctas;
+      launches += launch_fused_rkn(L, st);
+      for (size_t q = 0; q < group.p.size(); ++q) {
+        RunState& R = runs[q];
+        finish_device(C, *group.p[q], R);
+        launches += R.launches;
+        statuses.push_back(R.status);
+      }
+    }
     std::vector<unsigned> hs(4 * statuses.size() + 4, 0);
     for (size_t q = 0; q < statuses.size(); ++q)
       CK(cudaMemcpyAsync(&hs[4 * q], statuses[q], 16, cudaMemcpyDeviceToHost, st));
