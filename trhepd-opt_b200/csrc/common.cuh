@@ -39,6 +39,18 @@ __host__ __device__ __forceinline__ cd cdiv(cd a, cd b) {
     return cd{(a.x * r + a.y) / den, (a.y * r - a.x) / den};
   }
 }
+#ifdef __CUDACC__
+// 1 / d = conj(d) / |d|^2, d scaled by a power of two first: |d|^2 neither overflows nor
+// underflows, and the scaling rounds nothing.  One reciprocal, no branch (cdiv takes two
+// divisions and one).
+__device__ __forceinline__ cd crecip(cd d) {
+  const int e = max(__double2hiint(d.x) & 0x7fffffff, __double2hiint(d.y) & 0x7fffffff) >> 20;
+  const double s = __hiloint2double(max(2046 - e, 1) << 20, 0);  // 2^(1023 - e): 1 <= |s d| < 4
+  d = s * d;
+  const double r = __drcp_rn(fma(d.x, d.x, d.y * d.y));
+  return s * cd{d.x * r, -d.y * r};
+}
+#endif
 
 __host__ __device__ __forceinline__ int ceil_div(int a, int b) { return (a + b - 1) / b; }
 __host__ __device__ __forceinline__ int round_up(int a, int b) { return ceil_div(a, b) * b; }

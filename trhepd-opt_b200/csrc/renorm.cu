@@ -77,14 +77,6 @@ __device__ __forceinline__ void cp16(void* smem, const void* gmem, bool pred) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(gmem),
                "r"(pred ? 16 : 0));
 }
-// 1 / d by two Newton-Raphson steps y <- y + y (1 - d y) on the hardware's approximation
-// (about 2^-22): within an ulp or two, at a quarter of the division's latency.
-__device__ __forceinline__ double reciprocal(double d) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-  y = fma(y, fma(-d, y, 1.0), y);
-  return fma(y, fma(-d, y, 1.0), y);
-}
 
 // One cluster of `ctas` CTAs per angle.  kG = 1: CTA s holds the block's columns 16 s ..;
 // kG = 2 (the whole of [Q | P], c0 = 0, w = n): also P's columns 16 s .., and the
@@ -186,8 +178,7 @@ __global__ void __launch_bounds__(kMaxT, kMinB) k_gj_block(const BlockArgs g, in
           cd u[4];
 #pragma unroll
           for (int k = 0; k < 4; ++k) u[k] = up[((q + k) & 3) * 4 + t4];
-          const double dinv = reciprocal(fma(d.x, d.x, d.y * d.y));  // 1/d = conj(d) / |d|^2
-          const cd rc = cd{d.x * dinv, -d.y * dinv};
+          const cd rc = crecip(d);
 #pragma unroll
           for (int r = 0; r < kR; ++r) {
             // the row's entry of column jj is lane (gq, tj)'s

@@ -402,8 +402,7 @@ __global__ void __launch_bounds__(kThreads, Cfg<RT, GW, kRk4>::MINB)
           cd u[4];
 #pragma unroll
           for (int k = 0; k < 4; ++k) u[k] = urow[kb][k * 4 + t4];
-          const double dinv = 1.0 / (d.x * d.x + d.y * d.y);  // 1/d = conj(d) / |d|^2
-          const cd rc = cd{d.x * dinv, -d.y * dinv};
+          const cd rc = crecip(d);
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             const cd f = cd{__shfl_sync(full, x[h][q].x, tj, 4),
