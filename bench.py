@@ -6,15 +6,18 @@ bulk, N = 521 beams, 61 glancing angles (0.5..6.5 deg), 2004 slices of
 0.01 A, symplectic RKN-4 (int_method 5).  One step = one solve of all 61 angles.
 
 * ``value``: the split-precision form (``--precision`` bf16 / fp64 select the other
-  forms; beams on a dense index grid, as this workload's, take the FP64 convolution
-  stage products in every form, other beam sets 5 signed 8-bit digit slices per
-  operand on tcgen05 kind::i8), inputs resident in HBM
+  forms; beams on a dense index grid in thin slices, as this workload's, take the FP64
+  convolution stage products in every form, other beam sets 5 signed 8-bit digit slices
+  per operand on tcgen05 kind::i8: ``config.stage_products`` says which ran), inputs
+  resident in HBM
   (trhepd_problem_solve), device time from CUDA events on the library stream,
   max over ranks.
 * ``e2e``: the same metric through the C ABI with host buffers
   (trhepd_srfref: uploads, stage-table build, solve, intensities back).
 * ``fp64``: the plain FP64 form of the same workload, its speed and the split
-  form's error against it; ``bf16_split``: the BF16-slice form beside it.
+  form's error against it; ``bf16_split``: the BF16-slice form beside it (neither
+  where the main form ran the same FP64 kernels).
+* ``digit_products``: the INT8 and BF16 digit products on a beam set that takes them.
 * ``roofline``: the stage kernel, live event timing of every launch.
 * ``cpu_baseline``: the CPU oracle (C++ restatement of the reference path,
   OpenMP over angles, OpenBLAS) on a bounded sample of the workload.
@@ -366,6 +369,48 @@ def bulk_leg(ctx, cpu: bool) -> dict:
     return out
 
 
+def digit_leg(ctx, slices: int, n: int = 400, angles: int = 31) -> dict:
+    """The split forms where they run digit products: 400 beams on a 23 x 23 grid, sp4 at
+    0.02 A.  Device time of a solve, of one stage product and of its tcgen05 kernel, the
+    issued tensor rate and the error against the FP64 form of the same problem."""
+    out = {"nb": n, "nangles": angles, "digit_slices": slices}
+    try:
+        with tempfile.TemporaryDirectory() as d:
+            s = generator.dense(n, n_angles=angles, region=4.0, dz=0.02)
+            s.write(Path(d))
+            bulkfile.write_bulkp(s, Path(d) / "bulkP.b")
+            sp = surface.SurfaceProblem(ctx, Path(d) / "bulkP.b", Path(d) / "surf.txt",
+                                        s.surface_dz, s.int_method)
+        rp = sp.resident()
+        rp.solve(native.FP64)
+        _, ref = rp.fetch()
+        work = 8.0 * angles * n ** 3
+        for name, form in (("int8", native.SPLIT_INT8), ("bf16", native.SPLIT_BF16)):
+            if form == native.SPLIT_BF16 and slices > 5:
+                continue
+            for _ in range(3):
+                rp.solve(form)
+            ms = ctx.last_stats()["device_ms"]
+            _, f2 = rp.fetch()
+            ctx.set_option(native.OPT_PROFILE, 1)
+            rp.solve(form)
+            ctx.set_option(native.OPT_PROFILE, 0)
+            st = ctx.last_stats()
+            k = max(st["stage_products"], 1)
+            tensor = st["tensor_kernel_ms"] / k
+            rowmax = np.maximum(np.abs(ref).max(axis=1, keepdims=True), 1e-300)
+            out[name] = {"stages": st["stages"], "device_ms": ms,
+                         "angle_solves_per_s": angles / (ms / 1e3),
+                         "stage_product_ms": st["stage_kernel_ms"] / k, "kernel_ms": tensor,
+                         "issued_tops": slices * (slices + 1) // 2 * work / (tensor * 1e-3) / 1e12,
+                         "max_err_vs_rowmax": float((np.abs(f2 - ref) / rowmax).max())}
+        rp.close()
+        sp.close()
+    except Exception as e:  # a failed leg is reported, the bench line still prints
+        out["error"] = f"{type(e).__name__}: {e}"
+    return out
+
+
 def rk4_leg(ctx) -> dict:
     """int_method 7 (RK4, Gauss-Jordan renormalisation on the Gershgorin test) and
     int_method 8 (RK4, CholeskyQR when the power estimate exceeds 1e2) on the
@@ -411,6 +456,7 @@ def main():
     ap.add_argument("--no-serve", action="store_true")
     ap.add_argument("--no-uneven", action="store_true", help="skip the uneven candidate batch")
     ap.add_argument("--no-bulk", action="store_true", help="skip the bulk boundary solve leg")
+    ap.add_argument("--no-digits", action="store_true", help="skip the digit-product leg")
     ap.add_argument("--no-rk4", action="store_true", help="skip the int_method 7/8 leg")
     ap.add_argument("--uneven-per-n", type=int, default=64,
                     help="candidates per beam count in the uneven batch (64: 256 structures)")
@@ -513,8 +559,8 @@ def main():
     stp = solve_ms(prec)
     ctx.set_option(native.OPT_PROFILE, 0)
     nprod = max(stp["stage_products"], 1)
-    # a dense product takes a launch or more, the convolutions one for many stages
-    convolved = stp["launches"] < stp["stage_products"]
+    stages = stp["stages"]
+    convolved = stages == "convolution"  # in FP64, whatever the form
     tensor_ms = stp["tensor_kernel_ms"] / nprod
     stage_ms = stp["stage_kernel_ms"] / nprod
     fp64_equiv = 8.0 * nang * n ** 3  # complex N x N x N product per angle
@@ -563,7 +609,12 @@ def main():
         mma_issue = 2 * 8192 * sms * clk["sm_mhz"] * 1e6 / 1e12   # TOP/s
     traffic = NCU_TRAFFIC.get((args.workload, form, slices))
     tensor_floor_ms = issued / (peak * 1e12) * 1e3 if peak else 0.0
-    roof = convolution_roofline(stp, sp, nang, n, f64_peak) if convolved else {"bound": "tensor" if tensor_floor_ms >= hbm_ms else "hbm",
+    if stages == "convolution":
+        roof = convolution_roofline(stp, sp, nang, n, f64_peak)
+    elif stages == "fused":
+        roof = fused_roofline(stp, nang, n, f64_peak)
+    else:
+        roof = {"bound": "tensor" if tensor_floor_ms >= hbm_ms else "hbm",
             "achieved": achieved, "peak": peak, "unit": unit,
             "frac": (achieved / peak) if peak else None,
             "traffic": (traffic * nang / 16.0) if traffic else None,
@@ -615,7 +666,7 @@ def main():
 
     fp64 = None
     f2_64 = None
-    if split and not args.no_fp64:
+    if split and not convolved and not args.no_fp64:
         # the warm-up solve is profiled (per-launch events of the FP64 stage kernel),
         # the second one is timed without events
         ctx.set_option(native.OPT_PROFILE, 1)
@@ -625,8 +676,10 @@ def main():
         _, f2_64 = rp.fetch()
         fp64 = {"value": nang / (st["device_ms"] / 1e3), "ms_per_step": st["device_ms"],
                 "split_speedup": (st["device_ms"] / ms_per_step),
+                "stages": st64p["stages"],
                 "roofline": convolution_roofline(st64p, sp, nang, n, f64_peak)
-                if st64p["launches"] < st64p["stage_products"] else
+                if st64p["stages"] == "convolution" else
+                fused_roofline(st64p, nang, n, f64_peak) if st64p["stages"] == "fused" else
                 fp64_roofline(st64p, nang, n, f64_peak, peaks,
                               NCU_TRAFFIC.get((args.workload, "fp64", 0))),
                 "breakdown": {"solve_ms": st64p["device_ms"],
@@ -635,7 +688,7 @@ def main():
                               "renormalisations": st64p["renormalisations"]}}
         fp64.update({"split_" + k: v for k, v in errors(f2_main, f2_64).items()})
     bf16 = None
-    if prec == native.SPLIT_INT8 and not args.no_bf16:
+    if prec == native.SPLIT_INT8 and not convolved and not args.no_bf16:
         st, f2_b = compare(native.SPLIT_BF16)
         bf16 = {"value": nang / (st["device_ms"] / 1e3), "ms_per_step": st["device_ms"]}
         if f2_64 is not None:
@@ -675,6 +728,9 @@ def main():
     bulk = None
     if rank == 0 and ws == 1 and not args.no_bulk:
         bulk = bulk_leg(ctx, cpu=not args.no_cpu_baseline)
+    digits = None
+    if rank == 0 and ws == 1 and not args.no_digits:
+        digits = digit_leg(ctx, slices)
     rk4 = None
     if rank == 0 and ws == 1 and not args.no_rk4:
         rk4 = rk4_leg(ctx)
@@ -696,12 +752,17 @@ def main():
                                                   native.FP64: "f64"}[prec],
                 "data": "synthetic",
                 "config": {"workload": desc, "nb": n, "nangles": nang, "slices": rp.ns,
-                           "precision": {native.SPLIT_INT8: "split-int8",
-                                         native.SPLIT_BF16: "split-bf16",
-                                         native.FP64: "fp64"}[prec],
-                           "split_slices": slices if split else None,
-                           "stage_products": "FP64 convolutions over the beam grid" if convolved
-                           else "dense products",
+                           "precision": "fp64" if convolved else
+                           {native.SPLIT_INT8: "split-int8", native.SPLIT_BF16: "split-bf16",
+                            native.FP64: "fp64"}[prec],
+                           "precision_requested": {native.SPLIT_INT8: "split-int8",
+                                                   native.SPLIT_BF16: "split-bf16",
+                                                   native.FP64: "fp64"}[prec],
+                           "split_slices": slices if split and not convolved else None,
+                           "stage_products": {
+                               "convolution": "FP64 convolutions over the beam grid",
+                               "fused": "FP64, every stage in one launch",
+                               "dense": "dense products"}[stages],
                            "renormalisation": "growth bound ln(1e3)",
                            "renormalisations_per_solve": stp["renormalisations"],
                            "stage_products_per_solve": stp["stage_products"],
@@ -720,19 +781,43 @@ def main():
                 "serving": serve, "uneven_batch": uneven, "bulk_boundary": bulk,
                 "rk4_methods": rk4,
                 "breakdown": breakdown,
-                "bf16_split": bf16, "fp64": fp64,
+                "bf16_split": bf16, "fp64": fp64, "digit_products": digits,
                 # last, so that a truncated view of the line still shows them
                 "split_vs_fp64": None if not fp64 else {
                     "speedup": fp64["split_speedup"],
                     "max_rel_err_all_spots": fp64["split_max_rel_err_all_spots"],
                     "every_spot_within_1e-6": bool(fp64["split_max_rel_err_all_spots"] <= 1e-6),
                     "fp64_value": fp64["value"], "split_value": value,
-                    "renormalisation": "growth bound ln(1e3) and the same cluster elimination "
-                                       "on the FP64 tensor path for both forms"}}
+                    "renormalisation": "growth bound ln(1e3) for both forms"}}
         print(json.dumps(line), flush=True)
     if pg:
         pg.barrier()
         pg.destroy_process_group()
+
+
+def grid_span(sp, n: int) -> int:
+    """The smaller bounding grid's longer side of the beams' indices, sheared if that helps."""
+    import ctypes
+    ih, ik = (np.frombuffer(ctypes.string_at(p, 4 * n), np.int32)
+              for p in (sp.args.ih, sp.args.ik))
+    return 1 + min(max(int(np.ptp(a)), int(np.ptp(b + shear * a)))
+                   for shear in range(-2, 3) for a, b in ((ih, ik), (ik, ih)))
+
+
+def fused_roofline(stp: dict, nang: int, n: int, f64_peak) -> dict:
+    """Roofline of the fused small-beam kernel from one profiled solve: the complex
+    products, 8 n^3 per angle and stage, over the whole launch (its eliminations
+    included) against cuBLAS DGEMM measured in the run."""
+    work = 8.0 * nang * n ** 3 * max(stp["stage_products"], 1)
+    ms = stp["stage_kernel_ms"]
+    peak = f64_peak["sustained"] if f64_peak else None
+    achieved = work / (ms * 1e-3) / 1e12
+    return {"bound": "latency", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
+            "frac": achieved / peak if peak else None,
+            "kernel": "k_fused_rkn (FP64 DMMA, an angle per CTA, state in shared memory)",
+            "peak_source": "cuBLAS DGEMM 8192^3 measured in this run, sustained over a 3 s loop",
+            "launch_ms": ms, "stage_products": stp["stage_products"],
+            "ctas": nang, "note": "one CTA per angle: fewer than 148 angles leave SMs idle"}
 
 
 def convolution_roofline(stp: dict, sp, nang: int, n: int, f64_peak) -> dict:
@@ -742,18 +827,10 @@ def convolution_roofline(stp: dict, sp, nang: int, n: int, f64_peak) -> dict:
     turn, 10 per beam's update) against cuBLAS DGEMM measured in the run.  DFT arithmetic
     is half additions, so the FP64 pipe is fuller than the fraction says; the state stays
     on chip between renormalisations, so HBM does not bound it."""
-    import ctypes
     import math
 
-    def ints(ptr):
-        return np.frombuffer(ctypes.string_at(ptr, 4 * n), np.int32)
-    spans = []
-    for shear in range(-2, 3):
-        for a, b in ((ints(sp.args.ih), ints(sp.args.ik)), (ints(sp.args.ik), ints(sp.args.ih))):
-            v = b + shear * a
-            spans.append((max(int(np.ptp(a)), int(np.ptp(v))) + 1, int(np.ptp(a)) + 1))
-    span = min(spans)[0]
-    m = next(k for k in (9, 10, 12, 15, 16, 20, 25, 27, 32) if k >= span)
+    m = stp["transform_length"]
+    span = grid_span(sp, n)
     fft = 5.0 * m * math.log2(m)
     row = (4 * span + 8 * m) * fft + 6.0 * 4 * m * m + 6.0 * m * (2 * span + 4 * m) + 10.0 * n
     ms = stp["tensor_kernel_ms"] / max(stp["stage_products"], 1)

@@ -94,7 +94,10 @@ int trhepd_set_option(trhepd_context* ctx, int option, double value);
    out[5] kernels launched, out[6] of which renormalisation kernels, out[7] summed
    device milliseconds of the tensor-core kernel alone inside the stage products
    (TRHEPD_OPT_PROFILE only), out[8] summed device milliseconds of the end-of-slice
-   renormalisations (TRHEPD_OPT_PROFILE only) */
+   renormalisations (TRHEPD_OPT_PROFILE only), out[9] how the stages ran: 0 a dense
+   product each (digits in the split forms), 1 convolutions over the beam grid (FP64 in
+   every form), 2 the fused kernel, 3 several problems in a batch; out[10] the
+   convolutions' transform length.  At most n values are written. */
 int trhepd_last_stats(const trhepd_context* ctx, double* out, int n);
 /* Per-curve errors of the last validated split-form solve (TRHEPD_OPT_VALIDATE), one
    rocking curve per angle row: out[3a] = max over every spot of |I - I64| / |I64| (a

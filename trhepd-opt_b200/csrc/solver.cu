@@ -101,7 +101,7 @@ struct trhepd_context {
   int validate = 0;              // 1: split solves also run the FP64 form (per-curve errors)
   int particle = 0;              // trhepd_bulk_run: 0 positrons, 1 electrons
   int max_ctas = 0;              // persistent split kernels: CTA cap (0: one per SM, -1: one per tile)
-  double stats[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+  double stats[11] = {};
   std::vector<double> curve_err; // 3 per angle of the last validated solve (curves.h)
   std::vector<cudaEvent_t> evpool;
   std::vector<cudaEvent_t> rnpool;  // profile mode: pairs around renormalisations
@@ -230,6 +230,7 @@ struct RunState {
   StackedRows sr{};          // rows and stage-matrix stride per stacked problem
   int gj = kGjFp64, gj_edge = kGjFp64;  // renormalisations; boundary transforms
   bool conv = false;         // stage products as convolutions (convolve.h)
+  bool fused = false;        // the whole integration in one launch (small.h)
   ConvStages cs{};           // their constant arguments
   const int* centry = nullptr;
   cd* spec = nullptr;        // spectra of columns spec_col .. spec_col + spec_n - 1
@@ -770,6 +771,8 @@ void finish_host(trhepd_context* C, trhepd_problem& Pb, RunState& R) {
   C->stats[6] = (double)R.gj_launches;
   C->stats[7] = tensor_ms;
   C->stats[8] = renorm_ms;
+  C->stats[9] = R.conv ? 1.0 : R.fused ? 2.0 : 0.0;
+  C->stats[10] = R.conv ? (double)Pb.grid.m : 0.0;
   if (h_status[0] & kStatusTimeout) throw CudaError("device wait timed out", TRHEPD_ETIMEOUT);
   if (h_status[0] & (kStatusNonFinite | kStatusZeroPivot))
     throw CudaError("non-finite value or zero pivot in the surface solve", TRHEPD_ENONFINITE);
@@ -809,6 +812,7 @@ void fused_launch(trhepd_context* C, trhepd_problem& Pb, RunState& R,
   const cudaEvent_t* ev = C->profile ? &C->evpool[0] : nullptr;  // the launch is one entry
   for (int e = 0; ev && e < 2; ++e) CK(cudaEventRecord(ev[e], R.st));
   R.launches += launch(L, R.st);
+  R.fused = true;
   for (int e = 2; ev && e < 4; ++e) CK(cudaEventRecord(ev[e], R.st));
   if (ev) R.prof_entries = 1;
 }
@@ -1348,6 +1352,7 @@ void batch_solve(trhepd_context* C, trhepd_problem* const* probs, int count, int
     C->stats[1] = (double)products;
     C->stats[2] = ms;
     C->stats[5] = (double)launches;
+    C->stats[9] = 3.0;
   } catch (...) {
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
@@ -2087,7 +2092,7 @@ int trhepd_set_option(trhepd_context* c, int option, double value) {
 
 int trhepd_last_stats(const trhepd_context* c, double* out, int n) {
   if (!c || !out) return TRHEPD_EINVAL;
-  for (int i = 0; i < n && i < 9; ++i) out[i] = c->stats[i];
+  for (int i = 0; i < n && i < 11; ++i) out[i] = c->stats[i];
   return TRHEPD_OK;
 }
 

@@ -165,13 +165,15 @@ class Context:
         self._check(self._L.trhepd_set_option(self._h, option, float(value)))
 
     def last_stats(self) -> dict:
-        out = np.zeros(9)
-        self._check(self._L.trhepd_last_stats(self._h, out.ctypes.data, 9))
+        out = np.zeros(11)
+        self._check(self._L.trhepd_last_stats(self._h, out.ctypes.data, out.size))
         return {"renormalisations": int(out[0]), "stage_products": int(out[1]),
                 "device_ms": float(out[2]), "stage_columns": int(out[3]),
                 "stage_kernel_ms": float(out[4]), "launches": int(out[5]),
                 "renorm_launches": int(out[6]), "tensor_kernel_ms": float(out[7]),
-                "renorm_ms": float(out[8])}
+                "renorm_ms": float(out[8]),
+                "stages": ("dense", "convolution", "fused", "batch")[int(out[9])],
+                "transform_length": int(out[10])}
 
     def last_curve_errors(self, nangles: int) -> np.ndarray:
         """(nangles, 3) per-curve errors of the last validated split solve: max relative
