@@ -41,14 +41,24 @@ __host__ __device__ __forceinline__ cd cdiv(cd a, cd b) {
 }
 #ifdef __CUDACC__
 // 1 / d = conj(d) / |d|^2, d scaled by a power of two first: |d|^2 neither overflows nor
-// underflows, and the scaling rounds nothing.  One reciprocal, no branch (cdiv takes two
-// divisions and one).
+// underflows, and the scaling rounds nothing.  1 / |d|^2 by two Newton-Raphson steps
+// y <- y + y (1 - x y) on the hardware's approximation, good to its last bit or two where
+// x is a normal number, as it is here (2^-102 for the least subnormal d, else 1 to 8).
+// Each part to 6 * 2^-53.  Without a branch (cdiv: two divisions and one), and without a
+// call, around which the 96-register elimination spills: n = 95, 61 angles, 253 slices
+// take 63.2 ms with __drcp_rn, 61.4 so, 60.6 unscaled.
 __device__ __forceinline__ cd crecip(cd d) {
-  const int e = max(__double2hiint(d.x) & 0x7fffffff, __double2hiint(d.y) & 0x7fffffff) >> 20;
-  const double s = __hiloint2double(max(2046 - e, 1) << 20, 0);  // 2^(1023 - e): 1 <= |s d| < 4
+  constexpr int kExp = 0x7ff00000;  // the exponent's bits of the high word
+  const int e = max(__double2hiint(d.x) & kExp, __double2hiint(d.y) & kExp);
+  const double s = __hiloint2double(max(0x7fe00000 - e, 0x00100000), 0);
   d = s * d;
-  const double r = __drcp_rn(fma(d.x, d.x, d.y * d.y));
-  return s * cd{d.x * r, -d.y * r};
+  const cd ds = s * d;  // beside the chain of r: the scale of the result
+  const double x = fma(d.x, d.x, d.y * d.y);
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  r = fma(r, fma(-x, r, 1.0), r);
+  r = fma(r, fma(-x, r, 1.0), r);
+  return cd{ds.x * r, -ds.y * r};
 }
 #endif
 
