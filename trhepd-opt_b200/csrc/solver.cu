@@ -1353,6 +1353,7 @@ void batch_solve(trhepd_context* C, trhepd_problem* const* probs, int count, int
     C->stats[2] = ms;
     C->stats[5] = (double)launches;
     C->stats[9] = 3.0;
+    C->stats[10] = 0.0;
   } catch (...) {
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
