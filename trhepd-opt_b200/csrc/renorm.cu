@@ -537,31 +537,22 @@ __global__ void __launch_bounds__(256) k_gj_finish(const BlockArgs g) {
   }
 }
 
-// Rows of a warp and threads by n: 16 rows up to 128 (a cluster shares its SMs with
-// others), 32 up to 256, 48 up to 576 (at n = 521 eleven warps of 168 registers; 17
-// warps of 32 rows leave 96 registers and an uneven fifth warp on one scheduler).
-struct Shape {
-  int warp_rows, per_sm;  // per_sm: CTAs an SM holds
-};
-static Shape shape(int n) {
-  if (n <= 128) return {16, 4};
-  if (n <= 256) return {32, 2};
-  if (n <= 576) return {48, 1};
-  return {64, 1};
-}
 static bool whole(int n) { return n <= kMaxBlock * kW; }  // one launch
 
 // Sub-panels per block.  More of them means fewer passes over the trailing columns but
-// an SM each, idle while another's sub-panel is eliminated, so: six while all angles'
-// clusters fit about one wave, else four.  Whole elimination at n = 521 (one CTA per SM)
-// with 2 / 4 / 6 / 8 sub-panels per block: 1 angle 1.40 / 1.33 / 1.34 / 1.36 ms, 16
-// angles 3.22 / 2.72 / 2.55 / 2.79, 31 angles 4.95 / 4.07 / 4.44 / 4.87, 61 angles 8.28 /
-// 7.73 / 7.93 / 8.47 (now 1.21, 2.39, 3.74, 7.04; rank-32 updates with physical row swaps
-// and a launch per 16 columns took 4.2, 5.9, 6.8, 10.7 ms).
+// an SM each, idle while another's sub-panel is eliminated, so: six up to 18 angles,
+// else four.  Whole elimination at n = 521 (one CTA per SM) with 2 / 4 / 6 / 8 sub-panels
+// per block: 1 angle 1.40 / 1.33 / 1.34 / 1.36 ms, 16 angles 3.22 / 2.72 / 2.55 / 2.79, 31
+// angles 4.95 / 4.07 / 4.44 / 4.87, 61 angles 8.28 / 7.73 / 7.93 / 8.47 (now 1.22, 2.40,
+// 3.75, 7.10; rank-32 updates with physical row swaps and a launch per 16 columns took 4.2,
+// 5.9, 6.8, 10.7 ms).  The line holds from 150 to 600 beams, also where an SM takes two
+// CTAs: the time with four over that with six, at 16 / 24 / 31 / 61 angles: n = 150 1.02 /
+// 1.05 / 0.92 / 0.94, 191 1.05 / 0.90 / 0.94 / 0.86, 250 1.00 / 0.89 / 0.91 / 0.91, 400
+// 1.03 / 1.03 / 0.91 / 0.99, 600 1.02 / 0.92 / 0.87 / 0.92 (n = 191, 31 angles: 415 -> 390 us).
 static int block_ctas(int nang, int n) {
   const int sub = ceil_div(n, kW);
   if (whole(n)) return sub;
-  const int s = nang <= 18 * shape(n).per_sm ? 6 : 4;
+  const int s = nang <= 18 ? 6 : 4;
   return ceil_div(sub, ceil_div(sub, s));  // blocks of equal size
 }
 
@@ -644,6 +635,9 @@ int launch_gj_cluster(cd* Q, cd* P, const int* flag, int nang, int n, int ld, vo
     g.w = std::min(ctas * kW, n - c0);
     g.nsub = ceil_div(g.w, kW);
     g.ldc = round_up(2 * n - c0 - g.w, 4);
+    // rows of a warp: 16 up to 128 beams (above; a cluster shares its SMs with others), 32 up
+    // to 256, 48 up to 576 (at n = 521 eleven warps of 168 registers; 17 warps of 32 rows
+    // leave 96 registers and an uneven fifth warp on one scheduler)
     if (n <= 256) launch_block<1, 2, 256, 2>(g, nang, g.nsub, st);
     else if (n <= 576) launch_block<1, 3, 384, 1>(g, nang, g.nsub, st);
     else launch_block<1, 4, 320, 1>(g, nang, g.nsub, st);
