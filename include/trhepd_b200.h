@@ -34,7 +34,9 @@ enum trhepd_status {
 
 /* precision forms of the surface solve.  Where the beams lie on a dense index grid (nb >
    64) the stage products are FP64 convolutions in the FP64 form, and in the split forms
-   too where those are faster than their digit slices. */
+   too where those are faster than their digit slices and slices are thin (rms |gamma| dz
+   <= 3; int_method 7 and 8 in a split form always take digits).  Digit results repeat from
+   one build to another to the digits' truncation, not to FP64 rounding. */
 enum trhepd_precision {
   TRHEPD_FP64 = 0,        /* all-FP64 (DMMA) */
   TRHEPD_SPLIT_BF16 = 1,  /* stage products from BF16 slices on tcgen05 (FP32 accumulators),
@@ -68,15 +70,16 @@ enum trhepd_option {
                                    trhepd_problem_solve) is checked against the plain FP64 form
                                    of the same problem, solved first with the same options; the
                                    per-curve errors are read with trhepd_last_curve_errors.  Costs
-                                   one FP64 solve (about 3x the INT8 solve at N = 521) */
+                                   one FP64 solve (a few percent to 3 times the split solve) */
   TRHEPD_OPT_PARTICLE = 10,     /* trhepd_bulk_run: 0 positrons (TRHEPD, default), 1 electrons
                                    (RHEED): the program-level switch ep = 'P' / 'E' of bulk.exe
                                    (bulkm.f90:21-24), written to bulkP.b as inegpos; the surface
                                    solve follows the inegpos of the file it reads
                                    (surfio.f90:152) */
   TRHEPD_OPT_MAX_CTAS = 11      /* 0 (default): the stage-product kernels use every SM; k > 0:
-                                   the persistent split kernels run at most k CTAs and the FP64
-                                   stage kernel at most 2k blocks, leaving the other SMs to
+                                   the persistent split kernels run at most k CTAs, the FP64
+                                   stage kernel at most 2k blocks and the convolutions as many
+                                   as k SMs hold (2k to 8k), leaving the other SMs to
                                    kernels of other contexts (streams) on the same GPU; -1: the
                                    split kernels run one CTA per tile, so higher-priority work of
                                    other contexts starts between tiles */

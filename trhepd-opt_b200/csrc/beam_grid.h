@@ -66,10 +66,11 @@ inline ConvGrid conv_grid(int n, const int* ih, const int* ik, const int* pair) 
       m = l;
       break;
     }
-  // Below this filling the dense FP64 product is as fast: per row and stage the transforms
-  // take 5.3, 10.3, 20.3 and 21.2 ns at m = 15, 20, 25 and 27 whatever n is, the dense
-  // product about 3.5e-4 n^2 ns (n = 190 on a 25-grid: 14.5 against 20.2; n = 250: 25.0
-  // against 20.2).
+  // Below this filling the dense FP64 product may be as fast.  Thin-slice solves, us per
+  // stage, convolution / dense, 61 angles (m >= 25: 31): at the line m = 15, n = 92 28 / 50,
+  // m = 20, n = 162 95 / 145, m = 25, n = 252 159 / 199, m = 27, n = 293 195 / 341; at a
+  // filling of 0.32 (74 beams) 23 / 32, (130) 75 / 109, (202) 128 / 159, (235) 154 / 184; of
+  // 0.25 (102) 61 / 57, (158) 99 / 71, (184) 121 / 84.
   if (!m || (double)n < 0.4 * m * m) return g;
   g.sx = sx;
   g.sy = sy;

@@ -38,7 +38,8 @@ namespace {
 // per stage, us (threads x CTAs): n = 521, 31 angles: 313 (128 x 2), 323 (64 x 4), 343
 // (256 x 1), 377 (64 x 5, spills); n = 300, 61 angles: 163 / 217 / 185; n = 191, 61
 // angles: 54 (64 x 8), 58 (128 x 4), 74 (256 x 1); n = 95, 61 angles: 14.5 (96 x 5),
-// 16.2 (64 x 8), 18.4 (256 x 1); n = 70: 9.6 (128 x 5), 12.5 (256 x 1).
+// 16.2 (64 x 8), 18.4 (256 x 1); n = 70: 9.6 (128 x 5), 12.5 (256 x 1).  Launches of six
+// stages (an elimination after every slice) and slower machines of the kind: n = 191 62.
 template <int M>
 struct Shape {
   static constexpr int kThreads = M <= 10 ? 128 : M <= 12 ? 96 : M <= 16 ? 64 : 128;

@@ -478,11 +478,13 @@ bool rounding_amplified(const trhepd_problem& Pb, bool split) {
 
 // Whether the stage products of a solve are convolutions over the beam grid.  Against the
 // dense FP64 products they pay wherever conv_grid returns a grid (n = 521, 16 angles: 0.68
-// -> 0.17 ms per stage; n = 95, 61 angles: 56 -> 14.5 us).  Against the digit products (5
-// slices) they do on short transforms (n = 191, 61 angles, m = 15: 103 -> 62 us, 87 with 3
-// slices) and on well filled longer ones (31 angles, n = 521, m = 27: 376 -> 343 us; 61
-// angles, n = 300, m = 20: 225 -> 189), not below (n = 400, m = 25: 219 against 251; n = 250,
-// m = 25: 102 against 157) nor with fewer slices (n = 521, 4 slices: 330).
+// -> 0.17 ms per stage; n = 95, 61 angles: 56 -> 14.5 us).  Against the digit products they
+// do on short transforms, with any number of slices (us per stage of a thin-slice solve, 61
+// angles, 5 slices: n = 92 33 -> 28, n = 145 62 -> 46; 3 slices: n = 108 38 -> 34, n = 177
+// 76 -> 56), and with 5 slices on longer ones filled to 0.7 (digits / convolution: m = 20,
+// n = 288 208 / 176; m = 25, n = 441 306 / 297 at 31 angles and 567 / 577 at 61, n = 489 385 /
+// 336; m = 27, n = 515 442 / 378), not below (m = 20, n = 193 114 / 115; m = 25, n = 400 243 /
+// 264, n = 252 100 / 159) nor with fewer slices (n = 521, 31 angles, 4 slices: 330 / 343).
 bool use_convolution(const trhepd_context* C, const trhepd_problem& Pb, bool split) {
   const int m = Pb.grid.m;
   if (!m || Pb.I.family > kRk4 || rounding_amplified(Pb, split)) return false;
