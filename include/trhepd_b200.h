@@ -35,7 +35,7 @@ enum trhepd_status {
 /* precision forms of the surface solve.  Where the beams lie on a dense index grid (nb >
    64) the stage products are FP64 convolutions in the FP64 form, and in the split forms
    too where those are faster than their digit slices and slices are thin (rms |gamma| dz
-   <= 3; int_method 7 and 8 in a split form always take digits).  Digit results repeat from
+   <= 5; int_method 7 and 8 in a split form always take digits).  Digit results repeat from
    one build to another to the digits' truncation, not to FP64 rounding. */
 enum trhepd_precision {
   TRHEPD_FP64 = 0,        /* all-FP64 (DMMA) */

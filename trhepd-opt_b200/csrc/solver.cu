@@ -490,8 +490,10 @@ bool use_convolution(const trhepd_context* C, const trhepd_problem& Pb, bool spl
   if (!m || Pb.I.family > kRk4 || rounding_amplified(Pb, split)) return false;
   if (!split) return true;
   // the split forms' results stay those of the digits: their truncation, which the
-  // convolution does not have, is below 1e-11 of the curve up to here and 4e-9 at 8
-  if (Pb.gamma_rms * Pb.dz > 3.0) return false;
+  // convolution does not have, is 5e-12 of the curve at rms |gamma| dz = 4 (the most of 14
+  // sets), 2e-11 here, 6e-11 at 6, 7e-10 at 7.7 and 4e-9 at 8; the convolutions take a half
+  // to three quarters of the digits' time at 3 to 5
+  if (Pb.gamma_rms * Pb.dz > 5.0) return false;
   if (m <= 16) return true;
   return C->split_slices >= 5 && m <= 27 && (double)Pb.n >= 0.7 * m * m;
 }
